@@ -690,6 +690,12 @@ static int build_amg(sw2g_model* m) {
             g_err = "cudaMallocHost failed"; return SW2G_ERR_NOMEM;
         }
     }
+    if (A.lev[A.nlev - 1].n <= kAmgCoarsest) {   // the small levels in one cluster
+        const size_t rows = 3 * (size_t)A.lev[A.nlev - 1].n;
+        TRY(dalloc(m, &A.cl.op64, rows * rows)); TRY(dalloc(m, &A.cl.op32, rows * rows));
+        while (A.cl.lo < A.nlev - 1 && A.lev[A.cl.lo].n > kClusterNodes) A.cl.lo++;
+        A.cl.ctas = amg_cluster_ctas();
+    }
     m->amg_ready = true;
     static const bool trace = getenv("SW2G_TRACE_KRYLOV") != nullptr;
     if (trace) {
@@ -826,7 +832,11 @@ static int build_patches(sw2g_model* m, const double* vals) {
 // kernel launches of one preconditioner application (profiling counts)
 static int precond_launches(const sw2g_model* m, int precond) {
     if (precond == SW2G_PC_BILU0) return 2 * m->ilu.ncolors;
-    if (precond == SW2G_PC_AMG) return 1 + (m->amg.nlev - 1) * (2 * kAmgNu + 4) + 1 + 2;
+    if (precond == SW2G_PC_AMG) {   // per level: 2 kAmgNu sweeps, residual, restriction, prolongation
+        const AmgHost& H = m->amg;
+        const int lo = H.cl.ctas == 0 ? H.nlev - 1 : (H.cl.lo == 0 && H.patch.mode == 2) ? 1 : H.cl.lo;
+        return 1 + lo * (2 * kAmgNu + 3) + 1 + 2 * H.patch.mode;
+    }
     return 1;
 }
 

@@ -149,8 +149,16 @@ struct PatchDev {                           // device pointers (capacities kept 
     int mode = 0;                           // 0 off, 1 after each V-cycle, 2 inside it (after the level-0
                                             // pre-smoothing and after the post-smoothing)
 };
+// The small levels of a V-cycle in one thread-block cluster (amg_kernels.cu, k_amg_cluster).
+constexpr int kClusterNodes = 2048;         // levels of at most this many nodes
+struct ClusterPlan {
+    int ctas = 0;                           // CTAs of the cluster; 0: a kernel per pass and level
+    int lo = 0;                             // first level in the cluster
+    double* op64 = nullptr; float* op32 = nullptr;   // [(3n)^2] the coarsest level's operator, written by amg_setup
+};
 struct AmgHost {
     int nlev = 0;                       // levels including level 0
+    ClusterPlan cl;
     AmgLevel lev[kAmgMaxLevels];
     AmgLink link[kAmgMaxLevels];
     double* dinv0_64 = nullptr; float* dinv0_32 = nullptr;   // [9*nnodes] level-0 smoother blocks
@@ -161,6 +169,7 @@ template <> struct AmgBuf<double> {
     static const double* val(const AmgLevel& L) { return L.val64; }
     static const double* dinv(const AmgLevel& L) { return L.dinv64; }
     static const double* dinv0(const AmgHost& H) { return H.dinv0_64; }
+    static const double* coarsest(const AmgHost& H) { return H.cl.op64; }
     static double* b(const AmgLevel& L) { return L.b64; }
     static double* x(const AmgLevel& L) { return L.x64; }
     static double* t(const AmgLevel& L) { return L.t64; }
@@ -170,11 +179,13 @@ template <> struct AmgBuf<float> {
     static const float* val(const AmgLevel& L) { return L.val32; }
     static const float* dinv(const AmgLevel& L) { return L.dinv32; }
     static const float* dinv0(const AmgHost& H) { return H.dinv0_32; }
+    static const float* coarsest(const AmgHost& H) { return H.cl.op32; }
     static float* b(const AmgLevel& L) { return L.b32; }
     static float* x(const AmgLevel& L) { return L.x32; }
     static float* t(const AmgLevel& L) { return L.t32; }
     static float* r(const AmgLevel& L) { return L.r32; }
 };
+int amg_cluster_ctas();                     // CTAs of the cluster on the current device, 0: not available
 // numeric set-up from the scaled level-0 matrix (FP64, plus FP32 copies); writes H.patch.flag
 void amg_setup(const BlockCSR& A, const AmgHost& H, const AssemblyMaps& maps, const double* vals, cudaStream_t st);
 // inverts the chunk blocks of the current patch build (nchunks from the host build)
