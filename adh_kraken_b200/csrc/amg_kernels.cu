@@ -334,12 +334,6 @@ __global__ void __launch_bounds__(1024) k_amg_coarsest(int n, const int* __restr
     }
 }
 
-template <class VT>
-__global__ void k_amg_copy(int n, const VT* __restrict__ a, VT* __restrict__ b, const int* __restrict__ skip) {
-    if (skip && *skip) return;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) b[i] = a[i];
-}
-
 // ---------------------------------------------------------------- the small levels in one cluster
 // What bounds the small levels is latency, not bytes: each pass over a level of a few thousand
 // nodes is a handful of dependent L2 round trips (~280 cycles each), and as a launch of its own it
@@ -374,13 +368,15 @@ template <class VT> struct ClusterLevel {
     const int *bptr, *bcol;            // node graph (level 0: neighbour slots)
     const int *agg, *mptr, *mem;       // link to the next coarser level
     const VT *val, *dinv;              // level 0: values in the CSR layout
-    VT *b, *x, *t;
+    const VT* b;
+    VT *x, *t;
 };
 template <class VT> struct ClusterArgs {
     int lo, nlev;                      // levels lo .. nlev-1 run in the kernel
     const int* indptr0;                // CSR rows of level 0 (used when lo == 0)
     const int* skip;
     const VT* op;                      // the coarsest level's operator, row-major
+    VT* bc[kAmgMaxLevels];             // right-hand sides the kernel writes (levels past lo; the same as lev[l].b)
     ClusterLevel<VT> lev[kAmgMaxLevels];
 };
 struct Vec3 { double v0, v1, v2; };
@@ -493,7 +489,7 @@ __device__ __forceinline__ void cluster_down(const ClusterArgs<VT>& P, int l, do
     const int* ip = L0 ? P.indptr0 : nullptr;
     cluster_sweep<VT, L0, X_FIRST>(L, ip, nullptr, nullptr, L.x, w, gwarp, nwarps);
     cluster_sync();
-    cluster_restrict<VT, L0>(L, ip, P.lev[l + 1].n, P.lev[l + 1].b, gwarp, nwarps);
+    cluster_restrict<VT, L0>(L, ip, P.lev[l + 1].n, P.bc[l + 1], gwarp, nwarps);
     cluster_sync();
 }
 template <class VT, bool L0>
@@ -900,7 +896,7 @@ int amg_cluster_ctas() {
     return 0;
 }
 template <class VT>
-static void launch_cluster(const BlockCSR& A, const AmgHost& H, int lo, const VT* vals0, VT* b, VT* x, const int* skip,
+static void launch_cluster(const BlockCSR& A, const AmgHost& H, int lo, const VT* vals0, const VT* b, VT* x, const int* skip,
                            cudaStream_t st) {
     ClusterArgs<VT> P{};
     P.lo = lo; P.nlev = H.nlev; P.indptr0 = A.indptr; P.skip = skip; P.op = AmgBuf<VT>::coarsest(H);
@@ -910,7 +906,7 @@ static void launch_cluster(const BlockCSR& A, const AmgHost& H, int lo, const VT
         D.n = l ? L.n : A.nnodes;
         D.bptr = l ? L.bptr : A.bptr; D.bcol = l ? L.bcol : A.bcol;
         D.val = l ? AmgBuf<VT>::val(L) : vals0; D.dinv = l ? AmgBuf<VT>::dinv(L) : AmgBuf<VT>::dinv0(H);
-        D.b = AmgBuf<VT>::b(L); D.x = AmgBuf<VT>::x(L); D.t = AmgBuf<VT>::t(L);
+        D.b = P.bc[l] = AmgBuf<VT>::b(L); D.x = AmgBuf<VT>::x(L); D.t = AmgBuf<VT>::t(L);
         if (l + 1 < H.nlev) { D.agg = H.link[l].agg; D.mptr = H.link[l].mptr; D.mem = H.link[l].mem; }
     }
     P.lev[lo].b = b; P.lev[lo].x = x;
@@ -953,7 +949,7 @@ static void vcycle(const BlockCSR& A, const AmgHost& H, int l, const VT* vals0, 
     VT* t = AmgBuf<VT>::t(L);
     VT* r = AmgBuf<VT>::r(L);
     if (H.cl.ctas > 0 && l >= H.cl.lo && !(l == 0 && H.patch.mode == 2)) {   // (chunks inside the cycle: level 0 apart)
-        launch_cluster<VT>(A, H, l, vals0, const_cast<VT*>(b), x, skip, st);
+        launch_cluster<VT>(A, H, l, vals0, b, x, skip, st);
         return;
     }
     if (l == H.nlev - 1) {
@@ -984,7 +980,7 @@ static void vcycle(const BlockCSR& A, const AmgHost& H, int l, const VT* vals0, 
         cur = nxt;
     }
     if (l == 0 && H.patch.mode == 2) amg_patch_correct<VT>(A, H, vals0, b, cur, skip, st);
-    if (cur != x) k_amg_copy<VT><<<nb(3L * n, 256), 256, 0, st>>>(3 * n, cur, x, skip);
+    if (cur != x) copy_skip<VT>(3 * n, cur, x, skip, st);
 }
 
 void amg_smooth0_once(const BlockCSR& A, const AmgHost& H, const double* vals, const double* b, const double* x, double* y,
@@ -1003,11 +999,14 @@ template <class VT>
 void amg_patch_correct(const BlockCSR& A, const AmgHost& H, const VT* vals0, const VT* b, VT* y, const int* skip,
                        cudaStream_t st);
 template <class VT>
-void amg_apply(const BlockCSR& A, const AmgHost& H, const VT* vals0, VT* y, const int* skip, cudaStream_t st) {
-    VT* b0 = AmgBuf<VT>::b(H.lev[0]);
-    k_amg_copy<VT><<<1184, 256, 0, st>>>(3 * A.nnodes, y, b0, skip);
-    vcycle<VT>(A, H, 0, vals0, b0, y, skip, st);
-    if (H.patch.mode == 1) amg_patch_correct<VT>(A, H, vals0, b0, y, skip, st);
+void amg_apply(const BlockCSR& A, const AmgHost& H, const VT* vals0, const VT* x, VT* y, const int* skip, cudaStream_t st) {
+    if (x == y) {   // the cycle reads its right-hand side while it writes y
+        VT* b0 = AmgBuf<VT>::b(H.lev[0]);
+        copy_skip<VT>(3 * A.nnodes, x, b0, skip, st);
+        x = b0;
+    }
+    vcycle<VT>(A, H, 0, vals0, x, y, skip, st);
+    if (H.patch.mode == 1) amg_patch_correct<VT>(A, H, vals0, x, y, skip, st);
 }
 
 template <class VT>
@@ -1022,7 +1021,7 @@ template void amg_patch_correct<double>(const BlockCSR&, const AmgHost&, const d
                                         const int*, cudaStream_t);
 template void amg_patch_correct<float>(const BlockCSR&, const AmgHost&, const float*, const float*, float*,
                                        const int*, cudaStream_t);
-template void amg_apply<double>(const BlockCSR&, const AmgHost&, const double*, double*, const int*, cudaStream_t);
-template void amg_apply<float>(const BlockCSR&, const AmgHost&, const float*, float*, const int*, cudaStream_t);
+template void amg_apply<double>(const BlockCSR&, const AmgHost&, const double*, const double*, double*, const int*, cudaStream_t);
+template void amg_apply<float>(const BlockCSR&, const AmgHost&, const float*, const float*, float*, const int*, cudaStream_t);
 
 }  // namespace sw2

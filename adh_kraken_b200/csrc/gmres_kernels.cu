@@ -136,13 +136,6 @@ __global__ void k_gm_v0(int n, const VT* __restrict__ r, const double* __restric
         v0[i] = (VT)((double)r[i] * rw[i] * inv);
 }
 
-// w <- rw o w (row weights of the minimised residual norm)
-template <class VT>
-__global__ void k_gm_rowweight(int n, VT* __restrict__ w, const double* __restrict__ rw, GmresDev G) {
-    if (G.state[0]) return;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) w[i] = (VT)((double)w[i] * rw[i]);
-}
-
 // h_k = v_k . w for k < nv (w = v_nv before orthogonalisation), into column j of H.
 // blockIdx.y picks a group of kDotGroup basis vectors: each thread keeps kDotGroup
 // accumulators (about 40 registers instead of one per basis vector), so 6 blocks fit on
@@ -298,22 +291,28 @@ __global__ void __launch_bounds__(256) k_gm_orth(int n, int j, VT* __restrict__ 
         G.partial[blockIdx.x * (kGmM + 1)] = t;
     }
     if (!gm_last_block(G)) return;
-    const double tsum = gm_sum_partials(G, 0);
+    // the column and the earlier rotations in shared memory: one thread applies them in turn, and each step from
+    // global memory was an L2 round trip (8.7 us a launch at 30 columns on a small mesh)
+    __shared__ double cs[kGmM], sn[kGmM];
+    double* col = G.H + j * (kGmM + 1);
+    for (int k = threadIdx.x; k <= j; k += blockDim.x) {
+        if (SECOND) h[k] = __ldcg(col + k) + h[k];
+        if (k < j) { cs[k] = __ldcg(G.cs + k); sn[k] = __ldcg(G.sn + k); }
+    }
+    const double tsum = gm_sum_partials(G, 0);            // (synchronises the block)
     if (threadIdx.x == 0) {
         const double hn = sqrt(tsum);
-        double* col = G.H + j * (kGmM + 1);
-        if (SECOND)
-            for (int k = 0; k <= j; k++) col[k] += G.H2[k];
         for (int k = 0; k < j; k++) {                 // earlier rotations
-            const double a = col[k], b = col[k + 1];
-            col[k] = G.cs[k] * a + G.sn[k] * b;
-            col[k + 1] = -G.sn[k] * a + G.cs[k] * b;
+            const double a = h[k], b = h[k + 1];
+            h[k] = cs[k] * a + sn[k] * b;
+            h[k + 1] = -sn[k] * a + cs[k] * b;
         }
-        const double a = col[j], b = hn;
+        const double a = h[j], b = hn;
         const double rr = hypot(a, b);
         const double c = rr > 0.0 ? a / rr : 1.0, s = rr > 0.0 ? b / rr : 0.0;
         G.cs[j] = c; G.sn[j] = s;
-        col[j] = rr; col[j + 1] = 0.0;
+        h[j] = rr;
+        col[j + 1] = 0.0;
         G.g[j + 1] = -s * G.g[j];
         G.g[j] = c * G.g[j];
         G.scal[4] = hn;
@@ -323,6 +322,8 @@ __global__ void __launch_bounds__(256) k_gm_orth(int n, int j, VT* __restrict__ 
         else if (rr == 0.0) { G.state[2] = 1; G.state[0] = 1; G.state[1] = j; }   // breakdown: drop column j
         else if (!(fabs(G.g[j + 1]) > G.scal[1]) || hn == 0.0) G.state[0] = 1;
     }
+    __syncthreads();
+    for (int k = threadIdx.x; k <= j; k += blockDim.x) col[k] = h[k];
 }
 
 template <class VT>
@@ -333,30 +334,65 @@ __global__ void k_gm_scale(int n, int j, VT* __restrict__ Vb, size_t ld, GmresDe
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) w[i] = (VT)((double)w[i] * inv);
 }
 
-// y = H^-1 g on the k columns built (upper triangular after the rotations)
-__global__ void k_gm_solve(GmresDev G) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+// y = H^-1 g on the k columns built (upper triangular after the rotations).  One thread substitutes, in the order
+// of the columns; the rows it needs next are fetched into shared memory kSolveRows at a time by the block.
+constexpr int kSolveRows = 16;
+__global__ void __launch_bounds__(256) k_gm_solve(GmresDev G) {
+    __shared__ double rows[kSolveRows][kGmM], y[kGmM];
     const int k = G.state[1];
-    for (int i = k - 1; i >= 0; i--) {
-        double s = G.g[i];
-        for (int t = i + 1; t < k; t++) s -= G.H[t * (kGmM + 1) + i] * G.y[t];
-        const double d = G.H[i * (kGmM + 1) + i];
-        G.y[i] = d != 0.0 ? s / d : 0.0;
+    for (int top = k - 1; top >= 0; top -= kSolveRows) {
+        const int low = top - kSolveRows + 1 > 0 ? top - kSolveRows + 1 : 0;
+        __syncthreads();
+        for (int e = threadIdx.x; e < (top - low + 1) * k; e += blockDim.x) {
+            const int r = e % (top - low + 1), t = e / (top - low + 1);   // row low + r of column t
+            if (t >= low + r) rows[r][t] = G.H[t * (kGmM + 1) + low + r];
+        }
+        __syncthreads();
+        if (threadIdx.x == 0)
+            for (int i = top; i >= low; i--) {
+                double s = G.g[i];
+                for (int t = i + 1; t < k; t++) s -= rows[i - low][t] * y[t];
+                const double d = rows[i - low][i];
+                y[i] = d != 0.0 ? s / d : 0.0;
+            }
     }
-    G.state[0] = 0;   // let the final preconditioner apply run
+    __syncthreads();
+    for (int t = threadIdx.x; t < k; t += blockDim.x) G.y[t] = y[t];
+    if (threadIdx.x == 0) G.state[0] = 0;   // let the final preconditioner apply run
 }
 
-// out = V_k y
+// out = V_k y, 16 bytes per load and 8 basis vectors in flight (each entry's sum in basis order)
 template <class VT>
-__global__ void k_gm_combine(int n, const VT* __restrict__ Vb, size_t ld, VT* __restrict__ out, GmresDev G) {
+__global__ void __launch_bounds__(256) k_gm_combine(int n, const VT* __restrict__ Vb, size_t ld, VT* __restrict__ out, GmresDev G) {
     __shared__ double y[kGmM];
     const int k = G.state[1];
     for (int t = threadIdx.x; t < k; t += blockDim.x) y[t] = G.y[t];
     __syncthreads();
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        double s = 0;
-        for (int t = 0; t < k; t++) s += y[t] * (double)Vb[(size_t)t * ld + i];
-        out[i] = (VT)s;
+    constexpr int NQ = Quad<VT>::N;
+    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q * NQ < n; q += gridDim.x * blockDim.x) {
+        const size_t i = (size_t)q * NQ;          // the basis is padded to whole 16-byte pieces; out is not
+        double s[NQ];
+#pragma unroll
+        for (int c = 0; c < NQ; c++) s[c] = 0;
+        int t = 0;
+        for (; t + 8 <= k; t += 8) {
+            VT x[8][NQ];
+#pragma unroll
+            for (int u = 0; u < 8; u++) ld16(Vb + (size_t)(t + u) * ld + i, x[u]);
+#pragma unroll
+            for (int u = 0; u < 8; u++)
+#pragma unroll
+                for (int c = 0; c < NQ; c++) s[c] += y[t + u] * (double)x[u][c];
+        }
+        for (; t < k; t++) {
+            VT x[NQ];
+            ld16(Vb + (size_t)t * ld + i, x);
+#pragma unroll
+            for (int c = 0; c < NQ; c++) s[c] += y[t] * (double)x[c];
+        }
+#pragma unroll
+        for (int c = 0; c < NQ; c++)
+            if (i + c < (size_t)n) out[i + c] = (VT)s[c];
     }
 }
 
@@ -369,12 +405,8 @@ void gmres_cycle(const BlockCSR& A, const PrecondOp<VT>& P, const VT* vals, VT* 
     k_gm_v0<VT><<<g, 256, 0, st>>>(n, rhs, rw, Vb, G);
     if (m < 1 || m > kGmM) m = kGmM;
     for (int j = 0; j < m; j++) {
-        VT* vj = Vb + (size_t)j * ld;
-        VT* w = Vb + (size_t)(j + 1) * ld;
-        copy_skip<VT>(n, vj, z, done, st);
-        precond_apply<VT>(A, P, z, done, st);
-        spmv_skip<VT>(A, vals, z, w, done, st);
-        k_gm_rowweight<VT><<<g, 256, 0, st>>>(n, w, rw, G);
+        precond_apply<VT>(A, P, Vb + (size_t)j * ld, z, done, st);
+        spmv_skip<VT>(A, vals, z, Vb + (size_t)(j + 1) * ld, rw, done, st);
         const dim3 dg(g, (j + 1 + kDotGroup - 1) / kDotGroup);
         k_gm_dots<VT><<<dg, 256, 0, st>>>(n, j + 1, Vb, ld, G.H + (size_t)j * (kGmM + 1), G);
         if (reorth) {
@@ -386,9 +418,9 @@ void gmres_cycle(const BlockCSR& A, const PrecondOp<VT>& P, const VT* vals, VT* 
         }
         k_gm_scale<VT><<<g, 256, 0, st>>>(n, j, Vb, ld, G);
     }
-    k_gm_solve<<<1, 32, 0, st>>>(G);
-    k_gm_combine<VT><<<g, 256, 0, st>>>(n, Vb, ld, out, G);
-    precond_apply<VT>(A, P, out, nullptr, st);
+    k_gm_solve<<<1, 256, 0, st>>>(G);
+    k_gm_combine<VT><<<g, 256, 0, st>>>(n, Vb, ld, z, G);
+    precond_apply<VT>(A, P, z, out, nullptr, st);
 }
 template void gmres_cycle<double>(const BlockCSR&, const PrecondOp<double>&, const double*, double*, size_t, double*,
                                   const double*, double*, const double*, const GmresDev&, cudaStream_t, int, bool);

@@ -17,6 +17,7 @@
 //    bounds the partial arrays.
 #include <cmath>
 #include "sw2_launch.h"
+#include "sw2_reduce.cuh"
 
 namespace sw2 {
 
@@ -37,8 +38,6 @@ static int grid_for(long work, int threads) {
 }
 
 // ---------------------------------------------------------------- reductions
-__device__ __forceinline__ double ld_part(const Reduce& R, int i) { return __ldcg(R.partial + i); }
-
 template <int NT>
 __device__ __forceinline__ double block_sum(double v, double* sh) {
 #pragma unroll
@@ -63,8 +62,8 @@ __device__ __forceinline__ double block_max(double v, double* sh) {
     if (threadIdx.x == 0) for (int i = 0; i < NT / 32; i++) t = fmax(t, sh[i]);
     return t;
 }
-// Publish this block's partials; returns true in thread 0 of the last block, which
-// then reads every partial through ld_part (L1-bypassing loads).
+// Publish this block's partials; returns true in warp 0 of the last block, whose lanes then
+// reduce every block's partials (part_sum, part_max).
 __device__ __forceinline__ bool last_block(Reduce R, const double* vals, int nv) {
     __shared__ bool is_last;
     if (threadIdx.x == 0) {
@@ -74,8 +73,10 @@ __device__ __forceinline__ bool last_block(Reduce R, const double* vals, int nv)
         is_last = (t == gridDim.x - 1);
     }
     __syncthreads();
-    return is_last && threadIdx.x == 0;
+    return is_last && threadIdx.x < 32;
 }
+__device__ __forceinline__ double part_sum(const Reduce& R, int i) { return ordered_sum(R.partial + i, 4, (int)gridDim.x); }
+__device__ __forceinline__ double part_max(const Reduce& R, int i) { return warp_max(R.partial + i, 4, (int)gridDim.x); }
 
 // ---------------------------------------------------------------- Newton norms
 __global__ void __launch_bounds__(256) k_norms(int n, const double* __restrict__ res, const double* __restrict__ dsol,
@@ -92,11 +93,8 @@ __global__ void __launch_bounds__(256) k_norms(int n, const double* __restrict__
     double v[3];
     v[0] = block_max<256>(mx, sh); v[1] = block_sum<256>(l2, sh); v[2] = block_max<256>(im, sh);
     if (last_block(R, v, 3)) {
-        double a = 0, b = 0, c = 0;
-        for (int k = 0; k < (int)gridDim.x; k++) {
-            a = fmax(a, ld_part(R, 4 * k)); b += ld_part(R, 4 * k + 1); c = fmax(c, ld_part(R, 4 * k + 2));
-        }
-        R.out[0] = a; R.out[1] = b; R.out[2] = c;
+        const double a = part_max(R, 0), b = part_sum(R, 1), c = part_max(R, 2);
+        if (threadIdx.x == 0) { R.out[0] = a; R.out[1] = b; R.out[2] = c; }
     }
 }
 void launch_norms(int n, const double* res, const double* dsol, const int* bc_mask, Reduce R, cudaStream_t st) {
@@ -278,8 +276,8 @@ __global__ void __launch_bounds__(256) k_bicg_init2(BlockCSR A, KrylovVecs<VT> V
     double v[3];
     v[0] = block_max<256>(rmax, sh); v[1] = block_max<256>(bmax, sh); v[2] = block_sum<256>(rr, sh);
     if (last_block(R, v, 3)) {
-        double a = 0, b = 0, c = 0;
-        for (int k = 0; k < (int)gridDim.x; k++) { a = fmax(a, ld_part(R, 4 * k)); b = fmax(b, ld_part(R, 4 * k + 1)); c += ld_part(R, 4 * k + 2); }
+        const double a = part_max(R, 0), b = part_max(R, 1), c = part_sum(R, 2);
+        if (threadIdx.x) return;
         S->rnorm = a; S->bnorm = b; S->rho = c;
         S->rhop = 1.0; S->alpha = 1.0; S->omega = 1.0; S->beta = 0.0; S->it = 0; S->status = 0;
         S->done = (a > (S->tol + b * S->rtol)) ? 0 : 1;
@@ -309,8 +307,8 @@ __global__ void __launch_bounds__(256) k_bicg_spmv_p(BlockCSR A, KrylovVecs<VT> 
     double v[1];
     v[0] = block_sum<256>(qa, sh);
     if (last_block(R, v, 1)) {
-        double g = 0;
-        for (int k = 0; k < (int)gridDim.x; k++) g += ld_part(R, 4 * k);
+        const double g = part_sum(R, 0);
+        if (threadIdx.x) return;
         S->gamma = g;
         if (g == 0.0 || !isfinite(g)) { S->status = 1; S->done = 1; }
         else S->alpha = S->rho / g;
@@ -352,8 +350,8 @@ __global__ void __launch_bounds__(256) k_bicg_spmv_s(BlockCSR A, KrylovVecs<VT> 
     double v[3];
     v[0] = block_sum<256>(ss, sh); v[1] = block_sum<256>(aa, sh); v[2] = block_sum<256>(aq, sh);
     if (last_block(R, v, 3)) {
-        double a = 0, b = 0, c = 0;
-        for (int k = 0; k < (int)gridDim.x; k++) { a += ld_part(R, 4 * k); b += ld_part(R, 4 * k + 1); c += ld_part(R, 4 * k + 2); }
+        const double a = part_sum(R, 0), b = part_sum(R, 1), c = part_sum(R, 2);
+        if (threadIdx.x) return;
         if (b == 0.0) {            // s == 0: x + alpha p is the solution
             S->omega = 0.0; S->status = 3;
         } else {
@@ -392,8 +390,8 @@ __global__ void __launch_bounds__(256) k_bicg_update(int n, KrylovVecs<VT> V, Kr
     double v[1];
     v[0] = block_max<256>(rmax, sh);
     if (last_block(R, v, 1)) {
-        double m = 0;
-        for (int k = 0; k < (int)gridDim.x; k++) m = fmax(m, ld_part(R, 4 * k));
+        const double m = part_max(R, 0);
+        if (threadIdx.x) return;
         S->rnorm = m;
         S->it += 1;
         if (S->status == 3) { S->status = 0; S->done = 1; }
@@ -465,9 +463,8 @@ __global__ void __launch_bounds__(256) k_resid_pnorm(BlockCSR A, const double* _
     double v[1];
     v[0] = block_max<256>(zmax, sh);
     if (last_block(R, v, 1)) {
-        double mm = 0;
-        for (int k = 0; k < (int)gridDim.x; k++) mm = fmax(mm, ld_part(R, 4 * k));
-        R.out[0] = mm;
+        const double mm = part_max(R, 0);
+        if (threadIdx.x == 0) R.out[0] = mm;
     }
 }
 void launch_resid_pnorm(const BlockCSR& A, const double* vals, const double* inv, const double* x, const double* b,
@@ -544,9 +541,10 @@ int grid_resident(long work_items, int blocks_per_sm) {
     return (int)(need < cap ? need : cap);
 }
 
+// y = A x, or y = rw o (A x) with row weights (the residual norm GMRES minimises)
 template <class VT>
 __global__ void __launch_bounds__(256, kSweepBlocksPerSM) k_spmv(BlockCSR A, const VT* __restrict__ vals, const VT* __restrict__ x,
-                                              VT* __restrict__ y, const int* __restrict__ skip) {
+                                              VT* __restrict__ y, const double* __restrict__ rw, const int* __restrict__ skip) {
     if (skip && *skip) return;
     // lanes per node: 8 for FP64 values; 2 for FP32, whose half-size rows need more neighbour
     // blocks in flight per lane (the same choice as the AMG level-0 kernels, measured there)
@@ -577,7 +575,12 @@ __global__ void __launch_bounds__(256, kSweepBlocksPerSM) k_spmv(BlockCSR A, con
             y1 += __shfl_xor_sync(0xffffffffu, y1, o);
             y2 += __shfl_xor_sync(0xffffffffu, y2, o);
         }
-        if (g8 == 0 && valid) { y[3 * a] = (VT)y0; y[3 * a + 1] = (VT)y1; y[3 * a + 2] = (VT)y2; }
+        if (g8 == 0 && valid) {
+            if (rw) {   // the product rounded to VT, then its row weights, as two passes would
+                y0 = (double)(VT)y0 * rw[3 * a]; y1 = (double)(VT)y1 * rw[3 * a + 1]; y2 = (double)(VT)y2 * rw[3 * a + 2];
+            }
+            y[3 * a] = (VT)y0; y[3 * a + 1] = (VT)y1; y[3 * a + 2] = (VT)y2;
+        }
     }
 }
 // lanes per node of k_spmv (must match LANES inside it) and its one-wave grid
@@ -604,8 +607,8 @@ __global__ void __launch_bounds__(256) k_bicg_init_pc(int n, KrylovVecs<VT> V, K
     double v[3];
     v[0] = block_max<256>(rmax, sh); v[1] = block_max<256>(bmax, sh); v[2] = block_sum<256>(rr, sh);
     if (last_block(R, v, 3)) {
-        double a = 0, b = 0, c = 0;
-        for (int k = 0; k < (int)gridDim.x; k++) { a = fmax(a, ld_part(R, 4 * k)); b = fmax(b, ld_part(R, 4 * k + 1)); c += ld_part(R, 4 * k + 2); }
+        const double a = part_max(R, 0), b = part_max(R, 1), c = part_sum(R, 2);
+        if (threadIdx.x) return;
         S->rnorm = a; S->bnorm = b; S->rho = c;
         S->rhop = 1.0; S->alpha = 1.0; S->omega = 1.0; S->beta = 0.0; S->it = 0; S->status = 0;
         S->done = (a > (S->tol + b * S->rtol)) ? 0 : 1;
@@ -624,8 +627,8 @@ __global__ void __launch_bounds__(256) k_bicg_alpha(int n, KrylovVecs<VT> V, Kry
     double v[1];
     v[0] = block_sum<256>(qa, sh);
     if (last_block(R, v, 1)) {
-        double g = 0;
-        for (int k = 0; k < (int)gridDim.x; k++) g += ld_part(R, 4 * k);
+        const double g = part_sum(R, 0);
+        if (threadIdx.x) return;
         S->gamma = g;
         if (g == 0.0 || !isfinite(g)) { S->status = 1; S->done = 1; }
         else S->alpha = S->rho / g;
@@ -645,8 +648,8 @@ __global__ void __launch_bounds__(256) k_bicg_omega(int n, KrylovVecs<VT> V, Kry
     double v[3];
     v[0] = block_sum<256>(ss, sh); v[1] = block_sum<256>(aa, sh); v[2] = block_sum<256>(aq, sh);
     if (last_block(R, v, 3)) {
-        double a = 0, b = 0, c = 0;
-        for (int k = 0; k < (int)gridDim.x; k++) { a += ld_part(R, 4 * k); b += ld_part(R, 4 * k + 1); c += ld_part(R, 4 * k + 2); }
+        const double a = part_sum(R, 0), b = part_sum(R, 1), c = part_sum(R, 2);
+        if (threadIdx.x) return;
         if (b == 0.0) { S->omega = 0.0; S->status = 3; }
         else {
             const double om = a / b;
@@ -662,7 +665,7 @@ __global__ void __launch_bounds__(256) k_bicg_omega(int n, KrylovVecs<VT> V, Kry
 }
 
 void launch_spmv64(const BlockCSR& A, const double* vals, const double* x, double* y, cudaStream_t st) {
-    k_spmv<double><<<spmv_grid<double>(A.nnodes), 256, 0, st>>>(A, vals, x, y, nullptr);
+    k_spmv<double><<<spmv_grid<double>(A.nnodes), 256, 0, st>>>(A, vals, x, y, nullptr, nullptr);
 }
 
 template <class VT>
@@ -677,25 +680,27 @@ __global__ void k_uncast_skip(int n, const float* __restrict__ a, VT* __restrict
 }
 
 template <class VT>
-void precond_apply(const BlockCSR& A, const PrecondOp<VT>& P, VT* y, const int* skip, cudaStream_t st) {
+void precond_apply(const BlockCSR& A, const PrecondOp<VT>& P, const VT* x, VT* y, const int* skip, cudaStream_t st) {
     if (P.mixed) {
         PrecondOp<float> P32;
         P32.kind = P.kind; P32.ilu = P.ilu; P32.lu = P.lu32; P32.dinv = P.dinv32; P32.amg = P.amg; P32.vals = P.vals32;
         const int g = grid_for(A.n, 256);
-        k_cast_skip<VT><<<g, 256, 0, st>>>(A.n, y, P.tmp32, skip);
-        precond_apply<float>(A, P32, P.tmp32, skip, st);
+        float* in = P.kind == 2 ? AmgBuf<float>::b(P.amg->lev[0]) : P.tmp32;   // the cycle reads its own right-hand side
+        k_cast_skip<VT><<<g, 256, 0, st>>>(A.n, x, in, skip);
+        precond_apply<float>(A, P32, in, P.tmp32, skip, st);
         k_uncast_skip<VT><<<g, 256, 0, st>>>(A.n, P.tmp32, y, skip);
         return;
     }
     if (P.kind == 2) {
-        amg_apply<VT>(A, *P.amg, P.vals, y, skip, st);
+        amg_apply<VT>(A, *P.amg, P.vals, x, y, skip, st);
     } else {
+        if (x != y) copy_skip<VT>(A.n, x, y, skip, st);
         IluHost Hs = *P.ilu; Hs.view.skip = skip;
         launch_bilu_apply<VT>(A, Hs, P.lu, P.dinv, y, st);
     }
 }
-template void precond_apply<double>(const BlockCSR&, const PrecondOp<double>&, double*, const int*, cudaStream_t);
-template void precond_apply<float>(const BlockCSR&, const PrecondOp<float>&, float*, const int*, cudaStream_t);
+template void precond_apply<double>(const BlockCSR&, const PrecondOp<double>&, const double*, double*, const int*, cudaStream_t);
+template void precond_apply<float>(const BlockCSR&, const PrecondOp<float>&, const float*, float*, const int*, cudaStream_t);
 
 template <class VT>
 __global__ void k_copy_skip(int n, const VT* __restrict__ a, VT* __restrict__ b, const int* __restrict__ skip) {
@@ -716,14 +721,13 @@ void launch_bicg_init_pc(const BlockCSR& A, const PrecondOp<VT>& P, KrylovVecs<V
     const int gv = grid_for(A.n, 256);
     if (P.right) {
         k_copy<VT><<<gv, 256, 0, st>>>(A.n, V.b, V.x);                // y = b
-        k_copy<VT><<<gv, 256, 0, st>>>(A.n, V.x, V.z);
-        precond_apply<VT>(A, P, V.z, nullptr, st);                    // z = M^-1 y
-        k_spmv<VT><<<spmv_grid<VT>(A.nnodes), 256, 0, st>>>(A, V.vals, V.z, V.r, nullptr);
+        precond_apply<VT>(A, P, V.x, V.z, nullptr, st);               // z = M^-1 y
+        k_spmv<VT><<<spmv_grid<VT>(A.nnodes), 256, 0, st>>>(A, V.vals, V.z, V.r, nullptr, nullptr);
     } else {
-        precond_apply<VT>(A, P, V.b, nullptr, st);                    // b <- M^-1 b
+        precond_apply<VT>(A, P, V.b, V.b, nullptr, st);               // b <- M^-1 b
         k_copy<VT><<<gv, 256, 0, st>>>(A.n, V.b, V.x);                // x = b
-        k_spmv<VT><<<spmv_grid<VT>(A.nnodes), 256, 0, st>>>(A, V.vals, V.x, V.r, nullptr);
-        precond_apply<VT>(A, P, V.r, nullptr, st);                    // r <- M^-1 A x
+        k_spmv<VT><<<spmv_grid<VT>(A.nnodes), 256, 0, st>>>(A, V.vals, V.x, V.r, nullptr, nullptr);
+        precond_apply<VT>(A, P, V.r, V.r, nullptr, st);               // r <- M^-1 A x
     }
     k_bicg_init_pc<VT><<<gv, 256, 0, st>>>(A.n, V, S, R);
 }
@@ -732,13 +736,13 @@ void copy_skip(int n, const VT* a, VT* b, const int* skip, cudaStream_t st) {
     k_copy_skip<VT><<<grid_for(n, 256), 256, 0, st>>>(n, a, b, skip);
 }
 template <class VT>
-void spmv_skip(const BlockCSR& A, const VT* vals, const VT* x, VT* y, const int* skip, cudaStream_t st) {
-    k_spmv<VT><<<spmv_grid<VT>(A.nnodes), 256, 0, st>>>(A, vals, x, y, skip);
+void spmv_skip(const BlockCSR& A, const VT* vals, const VT* x, VT* y, const double* rw, const int* skip, cudaStream_t st) {
+    k_spmv<VT><<<spmv_grid<VT>(A.nnodes), 256, 0, st>>>(A, vals, x, y, rw, skip);
 }
 template void copy_skip<double>(int, const double*, double*, const int*, cudaStream_t);
 template void copy_skip<float>(int, const float*, float*, const int*, cudaStream_t);
-template void spmv_skip<double>(const BlockCSR&, const double*, const double*, double*, const int*, cudaStream_t);
-template void spmv_skip<float>(const BlockCSR&, const float*, const float*, float*, const int*, cudaStream_t);
+template void spmv_skip<double>(const BlockCSR&, const double*, const double*, double*, const double*, const int*, cudaStream_t);
+template void spmv_skip<float>(const BlockCSR&, const float*, const float*, float*, const double*, const int*, cudaStream_t);
 
 template <class VT>
 void launch_bicg_iteration_pc(const BlockCSR& A, const PrecondOp<VT>& P, KrylovVecs<VT> V, KrylovScalars* S, Reduce R,
@@ -746,22 +750,20 @@ void launch_bicg_iteration_pc(const BlockCSR& A, const PrecondOp<VT>& P, KrylovV
     const int gv = grid_for(A.n, 256), gs = spmv_grid<VT>(A.nnodes);
     const int* done = &S->done;
     if (P.right) {
-        k_copy_skip<VT><<<gv, 256, 0, st>>>(A.n, V.p, V.z, done);
-        precond_apply<VT>(A, P, V.z, done, st);
-        k_spmv<VT><<<gs, 256, 0, st>>>(A, V.vals, V.z, V.Ap, done);
+        precond_apply<VT>(A, P, V.p, V.z, done, st);
+        k_spmv<VT><<<gs, 256, 0, st>>>(A, V.vals, V.z, V.Ap, nullptr, done);
     } else {
-        k_spmv<VT><<<gs, 256, 0, st>>>(A, V.vals, V.p, V.Ap, done);
-        precond_apply<VT>(A, P, V.Ap, done, st);
+        k_spmv<VT><<<gs, 256, 0, st>>>(A, V.vals, V.p, V.Ap, nullptr, done);
+        precond_apply<VT>(A, P, V.Ap, V.Ap, done, st);
     }
     k_bicg_alpha<VT><<<gv, 256, 0, st>>>(A.n, V, S, R);
     k_bicg_s<VT><<<gv, 256, 0, st>>>(A.n, V, S);
     if (P.right) {
-        k_copy_skip<VT><<<gv, 256, 0, st>>>(A.n, V.s, V.z, done);
-        precond_apply<VT>(A, P, V.z, done, st);
-        k_spmv<VT><<<gs, 256, 0, st>>>(A, V.vals, V.z, V.As, done);
+        precond_apply<VT>(A, P, V.s, V.z, done, st);
+        k_spmv<VT><<<gs, 256, 0, st>>>(A, V.vals, V.z, V.As, nullptr, done);
     } else {
-        k_spmv<VT><<<gs, 256, 0, st>>>(A, V.vals, V.s, V.As, done);
-        precond_apply<VT>(A, P, V.As, done, st);
+        k_spmv<VT><<<gs, 256, 0, st>>>(A, V.vals, V.s, V.As, nullptr, done);
+        precond_apply<VT>(A, P, V.As, V.As, done, st);
     }
     k_bicg_omega<VT><<<gv, 256, 0, st>>>(A.n, V, S, R);
     k_bicg_update<VT><<<gv, 256, 0, st>>>(A.n, V, S, R);
@@ -829,8 +831,8 @@ __global__ void __launch_bounds__(256) k_maxabs(int n, const double* __restrict_
     double v[2];
     v[0] = block_max<256>(m, sh); v[1] = block_max<256>(bad, sh);
     if (last_block(R, v, 2)) {
-        double a = 0, b = 0;
-        for (int k = 0; k < (int)gridDim.x; k++) { a = fmax(a, ld_part(R, 4 * k)); b = fmax(b, ld_part(R, 4 * k + 1)); }
+        const double a = part_max(R, 0), b = part_max(R, 1);
+        if (threadIdx.x) return;
         R.out[0] = b > 0 ? NAN : a;   // a non-finite entry is reported, not hidden by fmax
     }
 }
@@ -845,8 +847,8 @@ __global__ void __launch_bounds__(256) k_maxabs_unscaled(int n, const double* __
     double v[2];
     v[0] = block_max<256>(m, sh); v[1] = block_max<256>(bad, sh);
     if (last_block(R, v, 2)) {
-        double a = 0, b = 0;
-        for (int k = 0; k < (int)gridDim.x; k++) { a = fmax(a, ld_part(R, 4 * k)); b = fmax(b, ld_part(R, 4 * k + 1)); }
+        const double a = part_max(R, 0), b = part_max(R, 1);
+        if (threadIdx.x) return;
         R.out[0] = b > 0 ? NAN : a;
     }
 }

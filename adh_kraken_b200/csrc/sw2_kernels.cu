@@ -18,6 +18,7 @@
 #include "sw2_element.cuh"
 #include "sw2_device.h"
 #include "sw2_launch.h"
+#include "sw2_reduce.cuh"
 
 namespace sw2 {
 
@@ -322,11 +323,9 @@ __global__ void __launch_bounds__(256) k_mass_balance(MeshView M, const double* 
         is_last = (t == gridDim.x - 1);
     }
     __syncthreads();
-    if (is_last && threadIdx.x == 0) {
-        double a = 0.0, b = 0.0;
-        for (int k = 0; k < (int)gridDim.x; k++) { a += __ldcg(partial + 4 * k); b += __ldcg(partial + 4 * k + 1); }
-        out[0] = a * density;
-        out[1] = b;
+    if (is_last && threadIdx.x < 32) {
+        const double a = ordered_sum(partial, 4, (int)gridDim.x), b = ordered_sum(partial + 1, 4, (int)gridDim.x);
+        if (threadIdx.x == 0) { out[0] = a * density; out[1] = b; }
     }
 }
 

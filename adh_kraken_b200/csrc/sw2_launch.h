@@ -195,9 +195,9 @@ void amg_smooth0_once(const BlockCSR& A, const AmgHost& H, const double* vals, c
                       cudaStream_t st);
 void amg_smooth0_once32(const BlockCSR& A, const AmgHost& H, const float* vals, const float* b, const float* x, float* y,
                         cudaStream_t st);
-// y <- V-cycle(y) followed by the chunk corrections; vals0 = the level-0 values in the Krylov precision
+// y <- V-cycle(x) followed by the chunk corrections (x may be y); vals0 = the level-0 values in the Krylov precision
 template <class VT>
-void amg_apply(const BlockCSR& A, const AmgHost& H, const VT* vals0, VT* y, const int* skip, cudaStream_t st);
+void amg_apply(const BlockCSR& A, const AmgHost& H, const VT* vals0, const VT* x, VT* y, const int* skip, cudaStream_t st);
 // y += the chunk corrections of the residual b - A y (the last stage of amg_apply)
 template <class VT>
 void amg_patch_correct(const BlockCSR& A, const AmgHost& H, const VT* vals0, const VT* b, VT* y, const int* skip,
@@ -216,8 +216,9 @@ struct PrecondOp {
     const float* vals32 = nullptr; const float* lu32 = nullptr; const float* dinv32 = nullptr;
     float* tmp32 = nullptr;             // [n] work vector
 };
+// y = M^-1 x (x may be y)
 template <class VT>
-void precond_apply(const BlockCSR& A, const PrecondOp<VT>& P, VT* y, const int* skip, cudaStream_t st);
+void precond_apply(const BlockCSR& A, const PrecondOp<VT>& P, const VT* x, VT* y, const int* skip, cudaStream_t st);
 
 // ---- restarted GMRES(m) cycle (gmres_kernels.cu)
 constexpr int kGmM = 200;               // largest Krylov dimension of one cycle (Hessenberg and partial buffers)
@@ -244,8 +245,9 @@ template <class VT>
 void copy_skip(int n, const VT* a, VT* b, const int* skip, cudaStream_t st);
 // max_i |t_i / s_i|: the unscaled residual of a scaled system (out[0] of R)
 void launch_maxabs_unscaled(int n, const double* t, const double* scale, Reduce R, cudaStream_t st);
+// y = A x, or rw o (A x) with row weights
 template <class VT>
-void spmv_skip(const BlockCSR& A, const VT* vals, const VT* x, VT* y, const int* skip, cudaStream_t st);
+void spmv_skip(const BlockCSR& A, const VT* vals, const VT* x, VT* y, const double* rw, const int* skip, cudaStream_t st);
 
 // BiCGStab with an explicit preconditioner apply: same scalars and stopping rule
 // as the fused block-Jacobi kernels above.
