@@ -223,9 +223,8 @@ static int l0_grid(int nnodes, int lanes) { return grid_resident((long)nnodes * 
 // with a grid of 8 blocks per SM: FP32 values 2 lanes (0.198 ms per sweep) vs 4 (0.226) vs 8
 // (0.265); FP64 4 lanes (0.304 ms) vs 8 (0.315).  Fewer lanes per node keep more independent
 // loads in flight per lane, which the latency-bound neighbour gathers need.  With the one-wave
-// grid (6 blocks per SM) the FP32 sweep takes 0.181 ms.
-template <class VT> struct L0Lanes { static constexpr int value = 4; };
-template <> struct L0Lanes<float> { static constexpr int value = 2; };
+// grid (6 blocks per SM) the FP32 sweep takes 0.181 ms.  (L0Lanes in sw2_launch.h; FP32 passes of large meshes run
+// tile_kernels.cu instead.)
 
 // Coarse levels (block CSR, 9 values per block), same modes, 8 lanes per row.
 template <class VT, int MODE>
@@ -923,8 +922,13 @@ static void launch_cluster(const BlockCSR& A, const AmgHost& H, int lo, const VT
 
 template <class VT>
 static void smooth_or_resid(const BlockCSR& A, const AmgLevel& L, int l, const VT* vals0, const VT* dinv, const VT* b,
-                            const VT* x, VT* y, bool resid, const int* skip, cudaStream_t st) {
-    if (l == 0) {
+                            const VT* x, VT* y, bool resid, int rev, const int* skip, cudaStream_t st) {
+    if (l == 0 && use_tiles<VT>(A)) {
+        if constexpr (sizeof(VT) == 4) {
+            if (resid) tile_resid(A, vals0, b, x, y, rev, skip, st);
+            else tile_sweep(A, vals0, dinv, b, x, y, kAmgOmega, rev, skip, st);
+        }
+    } else if (l == 0) {
         constexpr int LN = L0Lanes<VT>::value;
         if (resid) k_amg_l0<VT, 0, LN><<<l0_grid(A.nnodes, LN), 256, 0, st>>>(A, vals0, dinv, b, x, y, 0.0, skip);
         else k_amg_l0<VT, 1, LN><<<l0_grid(A.nnodes, LN), 256, 0, st>>>(A, vals0, dinv, b, x, y, kAmgOmega, skip);
@@ -959,24 +963,27 @@ static void vcycle(const BlockCSR& A, const AmgHost& H, int l, const VT* vals0, 
     }
     // pre-smoothing: the sweeps alternate between t and x so that the last lands in x
     VT* cur = (kAmgNu % 2 == 1) ? x : t;
+    // direction of the level-0 passes: alternating, and forward in the matrix product between two cycles
+    static_assert(2 * kAmgNu % 2 == 0, "an even number of matrix passes a cycle");
+    int rev = 0;
     k_amg_scale<VT><<<nb(n, 256), 256, 0, st>>>(n, dinv, b, cur, kAmgOmega, skip);
     for (int s = 1; s < kAmgNu; s++) {
         VT* nxt = (cur == x) ? t : x;
-        smooth_or_resid<VT>(A, L, l, vals0, dinv, b, cur, nxt, false, skip, st);
+        smooth_or_resid<VT>(A, L, l, vals0, dinv, b, cur, nxt, false, rev ^= 1, skip, st);
         cur = nxt;
     }
     if (l == 0 && H.patch.mode == 2) amg_patch_correct<VT>(A, H, vals0, b, cur, skip, st);
     // coarse correction
     const AmgLevel& C = H.lev[l + 1];
     const AmgLink& K = H.link[l];
-    smooth_or_resid<VT>(A, L, l, vals0, dinv, b, cur, r, true, skip, st);
+    smooth_or_resid<VT>(A, L, l, vals0, dinv, b, cur, r, true, rev ^= 1, skip, st);
     k_amg_restrict<VT><<<nb(C.n, 128), 128, 0, st>>>(C.n, K.mptr, K.mem, r, AmgBuf<VT>::b(C), skip);
     vcycle<VT>(A, H, l + 1, vals0, AmgBuf<VT>::b(C), AmgBuf<VT>::x(C), skip, st);
     k_amg_prolong<VT><<<nb(3L * n, 256), 256, 0, st>>>(3 * n, K.agg, AmgBuf<VT>::x(C), cur, skip);
     // post-smoothing
     for (int s = 0; s < kAmgNu; s++) {
         VT* nxt = (cur == x) ? t : x;
-        smooth_or_resid<VT>(A, L, l, vals0, dinv, b, cur, nxt, false, skip, st);
+        smooth_or_resid<VT>(A, L, l, vals0, dinv, b, cur, nxt, false, rev ^= 1, skip, st);
         cur = nxt;
     }
     if (l == 0 && H.patch.mode == 2) amg_patch_correct<VT>(A, H, vals0, b, cur, skip, st);
@@ -985,14 +992,12 @@ static void vcycle(const BlockCSR& A, const AmgHost& H, int l, const VT* vals0, 
 
 void amg_smooth0_once(const BlockCSR& A, const AmgHost& H, const double* vals, const double* b, const double* x, double* y,
                       cudaStream_t st) {
-    constexpr int LN = L0Lanes<double>::value;
-    k_amg_l0<double, 1, LN><<<l0_grid(A.nnodes, LN), 256, 0, st>>>(A, vals, H.dinv0_64, b, x, y, kAmgOmega, nullptr);
+    smooth_or_resid<double>(A, H.lev[0], 0, vals, H.dinv0_64, b, x, y, false, 0, nullptr, st);
 }
 
 void amg_smooth0_once32(const BlockCSR& A, const AmgHost& H, const float* vals, const float* b, const float* x, float* y,
                         cudaStream_t st) {
-    constexpr int LN = L0Lanes<float>::value;
-    k_amg_l0<float, 1, LN><<<l0_grid(A.nnodes, LN), 256, 0, st>>>(A, vals, H.dinv0_32, b, x, y, kAmgOmega, nullptr);
+    smooth_or_resid<float>(A, H.lev[0], 0, vals, H.dinv0_32, b, x, y, false, 0, nullptr, st);
 }
 
 template <class VT>

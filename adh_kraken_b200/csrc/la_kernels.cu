@@ -548,7 +548,7 @@ __global__ void __launch_bounds__(256, kSweepBlocksPerSM) k_spmv(BlockCSR A, con
     if (skip && *skip) return;
     // lanes per node: 8 for FP64 values; 2 for FP32, whose half-size rows need more neighbour
     // blocks in flight per lane (the same choice as the AMG level-0 kernels, measured there)
-    constexpr int LANES = sizeof(VT) == 4 ? 2 : 8, PER_WARP = 32 / LANES;
+    constexpr int LANES = SpmvLanes<VT>::value, PER_WARP = 32 / LANES;
     const int g8 = threadIdx.x & (LANES - 1), sub = (threadIdx.x & 31) / LANES;
     const int nw = (gridDim.x * blockDim.x) >> 5;
     for (int base = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * PER_WARP; base < A.nnodes; base += nw * PER_WARP) {
@@ -583,9 +583,12 @@ __global__ void __launch_bounds__(256, kSweepBlocksPerSM) k_spmv(BlockCSR A, con
         }
     }
 }
-// lanes per node of k_spmv (must match LANES inside it) and its one-wave grid
-template <class VT> static int spmv_grid(int nnodes) {
-    return grid_resident((long)nnodes * (sizeof(VT) == 4 ? 2 : 8), kSweepBlocksPerSM);
+template <class VT>
+static void run_spmv(const BlockCSR& A, const VT* vals, const VT* x, VT* y, const double* rw, const int* skip, cudaStream_t st) {
+    if constexpr (sizeof(VT) == 4)
+        if (use_tiles<VT>(A)) { tile_product(A, vals, x, y, rw, 0, skip, st); return; }
+    // a one-wave grid
+    k_spmv<VT><<<grid_resident((long)A.nnodes * SpmvLanes<VT>::value, kSweepBlocksPerSM), 256, 0, st>>>(A, vals, x, y, rw, skip);
 }
 
 template <class VT>
@@ -665,7 +668,7 @@ __global__ void __launch_bounds__(256) k_bicg_omega(int n, KrylovVecs<VT> V, Kry
 }
 
 void launch_spmv64(const BlockCSR& A, const double* vals, const double* x, double* y, cudaStream_t st) {
-    k_spmv<double><<<spmv_grid<double>(A.nnodes), 256, 0, st>>>(A, vals, x, y, nullptr, nullptr);
+    run_spmv<double>(A, vals, x, y, nullptr, nullptr, st);
 }
 
 template <class VT>
@@ -722,11 +725,11 @@ void launch_bicg_init_pc(const BlockCSR& A, const PrecondOp<VT>& P, KrylovVecs<V
     if (P.right) {
         k_copy<VT><<<gv, 256, 0, st>>>(A.n, V.b, V.x);                // y = b
         precond_apply<VT>(A, P, V.x, V.z, nullptr, st);               // z = M^-1 y
-        k_spmv<VT><<<spmv_grid<VT>(A.nnodes), 256, 0, st>>>(A, V.vals, V.z, V.r, nullptr, nullptr);
+        run_spmv<VT>(A, V.vals, V.z, V.r, nullptr, nullptr, st);
     } else {
         precond_apply<VT>(A, P, V.b, V.b, nullptr, st);               // b <- M^-1 b
         k_copy<VT><<<gv, 256, 0, st>>>(A.n, V.b, V.x);                // x = b
-        k_spmv<VT><<<spmv_grid<VT>(A.nnodes), 256, 0, st>>>(A, V.vals, V.x, V.r, nullptr, nullptr);
+        run_spmv<VT>(A, V.vals, V.x, V.r, nullptr, nullptr, st);
         precond_apply<VT>(A, P, V.r, V.r, nullptr, st);               // r <- M^-1 A x
     }
     k_bicg_init_pc<VT><<<gv, 256, 0, st>>>(A.n, V, S, R);
@@ -737,7 +740,7 @@ void copy_skip(int n, const VT* a, VT* b, const int* skip, cudaStream_t st) {
 }
 template <class VT>
 void spmv_skip(const BlockCSR& A, const VT* vals, const VT* x, VT* y, const double* rw, const int* skip, cudaStream_t st) {
-    k_spmv<VT><<<spmv_grid<VT>(A.nnodes), 256, 0, st>>>(A, vals, x, y, rw, skip);
+    run_spmv<VT>(A, vals, x, y, rw, skip, st);
 }
 template void copy_skip<double>(int, const double*, double*, const int*, cudaStream_t);
 template void copy_skip<float>(int, const float*, float*, const int*, cudaStream_t);
@@ -747,22 +750,22 @@ template void spmv_skip<float>(const BlockCSR&, const float*, const float*, floa
 template <class VT>
 void launch_bicg_iteration_pc(const BlockCSR& A, const PrecondOp<VT>& P, KrylovVecs<VT> V, KrylovScalars* S, Reduce R,
                               cudaStream_t st) {
-    const int gv = grid_for(A.n, 256), gs = spmv_grid<VT>(A.nnodes);
+    const int gv = grid_for(A.n, 256);
     const int* done = &S->done;
     if (P.right) {
         precond_apply<VT>(A, P, V.p, V.z, done, st);
-        k_spmv<VT><<<gs, 256, 0, st>>>(A, V.vals, V.z, V.Ap, nullptr, done);
+        run_spmv<VT>(A, V.vals, V.z, V.Ap, nullptr, done, st);
     } else {
-        k_spmv<VT><<<gs, 256, 0, st>>>(A, V.vals, V.p, V.Ap, nullptr, done);
+        run_spmv<VT>(A, V.vals, V.p, V.Ap, nullptr, done, st);
         precond_apply<VT>(A, P, V.Ap, V.Ap, done, st);
     }
     k_bicg_alpha<VT><<<gv, 256, 0, st>>>(A.n, V, S, R);
     k_bicg_s<VT><<<gv, 256, 0, st>>>(A.n, V, S);
     if (P.right) {
         precond_apply<VT>(A, P, V.s, V.z, done, st);
-        k_spmv<VT><<<gs, 256, 0, st>>>(A, V.vals, V.z, V.As, nullptr, done);
+        run_spmv<VT>(A, V.vals, V.z, V.As, nullptr, done, st);
     } else {
-        k_spmv<VT><<<gs, 256, 0, st>>>(A, V.vals, V.s, V.As, nullptr, done);
+        run_spmv<VT>(A, V.vals, V.s, V.As, nullptr, done, st);
         precond_apply<VT>(A, P, V.As, V.As, done, st);
     }
     k_bicg_omega<VT><<<gv, 256, 0, st>>>(A.n, V, S, R);
