@@ -1,5 +1,5 @@
 // One cycle of right-preconditioned GMRES(m) on the scaled SW2 system, entirely
-// on the device so that a cycle is one CUDA graph replay.
+// on the device, so that a cycle is a few CUDA graph replays (kGmSegment steps each).
 //
 // Why next to the reference's BiCGStab: with an approximate multilevel
 // preconditioner the preconditioned SW2 operator at large Courant numbers is far
@@ -397,14 +397,17 @@ __global__ void __launch_bounds__(256) k_gm_combine(int n, const VT* __restrict_
 }
 
 template <class VT>
-void gmres_cycle(const BlockCSR& A, const PrecondOp<VT>& P, const VT* vals, VT* Vb, size_t ld, VT* z, const VT* rhs,
-                 VT* out, const double* rw, const GmresDev& G, cudaStream_t st, int m, bool reorth) {
-    const int n = A.n, g = gm_grid(n);
-    const int* done = G.state;
+void gmres_begin(int n, VT* Vb, const VT* rhs, const double* rw, const GmresDev& G, cudaStream_t st) {
+    const int g = gm_grid(n);
     k_gm_start<VT><<<g, 256, 0, st>>>(n, rhs, rw, G);
     k_gm_v0<VT><<<g, 256, 0, st>>>(n, rhs, rw, Vb, G);
-    if (m < 1 || m > kGmM) m = kGmM;
-    for (int j = 0; j < m; j++) {
+}
+template <class VT>
+void gmres_steps(const BlockCSR& A, const PrecondOp<VT>& P, const VT* vals, VT* Vb, size_t ld, VT* z, const double* rw,
+                 const GmresDev& G, cudaStream_t st, int first, int last, bool reorth) {
+    const int n = A.n, g = gm_grid(n);
+    const int* done = G.state;
+    for (int j = first; j < last; j++) {
         precond_apply<VT>(A, P, Vb + (size_t)j * ld, z, done, st);
         spmv_skip<VT>(A, vals, z, Vb + (size_t)(j + 1) * ld, rw, done, st);
         const dim3 dg(g, (j + 1 + kDotGroup - 1) / kDotGroup);
@@ -418,13 +421,19 @@ void gmres_cycle(const BlockCSR& A, const PrecondOp<VT>& P, const VT* vals, VT* 
         }
         k_gm_scale<VT><<<g, 256, 0, st>>>(n, j, Vb, ld, G);
     }
+}
+template <class VT>
+void gmres_end(const BlockCSR& A, const PrecondOp<VT>& P, VT* Vb, size_t ld, VT* z, VT* out, const GmresDev& G, cudaStream_t st) {
     k_gm_solve<<<1, 256, 0, st>>>(G);
-    k_gm_combine<VT><<<g, 256, 0, st>>>(n, Vb, ld, z, G);
+    k_gm_combine<VT><<<gm_grid(A.n), 256, 0, st>>>(A.n, Vb, ld, z, G);
     precond_apply<VT>(A, P, z, out, nullptr, st);
 }
-template void gmres_cycle<double>(const BlockCSR&, const PrecondOp<double>&, const double*, double*, size_t, double*,
-                                  const double*, double*, const double*, const GmresDev&, cudaStream_t, int, bool);
-template void gmres_cycle<float>(const BlockCSR&, const PrecondOp<float>&, const float*, float*, size_t, float*,
-                                 const float*, float*, const double*, const GmresDev&, cudaStream_t, int, bool);
+#define SW2_GMRES_INSTANCE(VT)                                                                                             \
+    template void gmres_begin<VT>(int, VT*, const VT*, const double*, const GmresDev&, cudaStream_t);                      \
+    template void gmres_steps<VT>(const BlockCSR&, const PrecondOp<VT>&, const VT*, VT*, size_t, VT*, const double*,       \
+                                  const GmresDev&, cudaStream_t, int, int, bool);                                          \
+    template void gmres_end<VT>(const BlockCSR&, const PrecondOp<VT>&, VT*, size_t, VT*, VT*, const GmresDev&, cudaStream_t);
+SW2_GMRES_INSTANCE(double)
+SW2_GMRES_INSTANCE(float)
 
 }  // namespace sw2

@@ -46,6 +46,23 @@ static const double kPatchTileEdges = 7.0;   // tile side of the AMG chunk corre
 
 struct ProfRec { int cls; cudaEvent_t a, b; };
 
+// A GMRES cycle as captured graphs: segments of kGmSegment steps (the first with the cycle's start) and the end.  The
+// host looks at the stop flag between segments, so that a cycle that converges early does not replay the steps
+// left as empty launches: those were 400 of 600 steps of a 125k-triangle solve with GMRES(100), 1.3 us a launch, 10 of
+// 49 ms; a look costs ~15 us.  Cycles of up to kGmSegment + 7 steps stay whole.
+static const int kGmSegment = 25;
+struct CycleGraph {
+    std::vector<cudaGraphExec_t> seg;
+    cudaGraphExec_t end = nullptr;
+    int m = 0, precond = -1;           // restart length and preconditioner it was built for
+    int per_segment = 0;               // steps of a segment (the last may have fewer)
+    void clear() {
+        for (cudaGraphExec_t g : seg) cudaGraphExecDestroy(g);
+        if (end) cudaGraphExecDestroy(end);
+        seg.clear(); end = nullptr; m = 0;
+    }
+};
+
 struct sw2g_model {
     int V = 0, T = 0, S = 0, Etot = 0, n = 0, nnz = 0, nslots = 0;
     int device = 0;   // the device current at sw2g_create: every buffer and the stream live there
@@ -77,7 +94,7 @@ struct sw2g_model {
     // reductions / scalars
     double *d_partial = nullptr, *d_rout = nullptr; unsigned int* d_counter = nullptr;
     KrylovScalars* d_ks = nullptr;
-    double* h_rout = nullptr; KrylovScalars* h_ks = nullptr;
+    double* h_rout = nullptr; KrylovScalars* h_ks = nullptr; int* h_state = nullptr;   // pinned
     cudaGraphExec_t graph64[3] = {nullptr, nullptr, nullptr}, graph32[3] = {nullptr, nullptr, nullptr};   // [precond]
     // multicolour block ILU(0)
     std::vector<int> h_color_ptr;
@@ -92,10 +109,8 @@ struct sw2g_model {
     double* gm_V64 = nullptr;            // [cap+1][gm_ld(n)] Krylov basis
     float* gm_V32 = nullptr;             // [cap+1][gm_ld(n)] FP32 Krylov basis (krylov_basis_precision 32)
     int gm_cap64 = 0, gm_cap32 = 0;      // restart length the bases were allocated for
-    cudaGraphExec_t gm_graph_b32 = nullptr;
-    int gm_m64 = 0, gm_m32 = 0, gm_mb32 = 0;   // restart length each cycle graph was built for
+    CycleGraph gm_cycle64, gm_cycle32, gm_cycle_b32;   // FP64, FP32 preconditioner, FP32 throughout
     double* gm_rw = nullptr;             // [n] row weights 1/s: GMRES minimises the unscaled residual
-    cudaGraphExec_t gm_graph64 = nullptr, gm_graph32 = nullptr;
     std::vector<int> h_bptr, h_bcol;   // node graph, kept for the AMG set-up
     // chunk corrections of the AMG (built every Newton iteration from the flagged nodes)
     std::vector<long long> h_tile;     // [V] tile of each node (squares of kPatchTileEdges mean edge lengths)
@@ -400,7 +415,8 @@ extern "C" int sw2g_create(const sw2g_mesh* mesh, void* cuda_stream, sw2g_model*
     CK(cudaMemsetAsync(m->d_EJ, 0, sizeof(double) * 81 * (size_t)m->Etot, m->st));
     CK(cudaMemsetAsync(m->d_ER, 0, sizeof(double) * 9 * (size_t)m->Etot, m->st));
     if (cudaMallocHost((void**)&m->h_rout, 8 * sizeof(double)) != cudaSuccess ||
-        cudaMallocHost((void**)&m->h_ks, sizeof(KrylovScalars)) != cudaSuccess) {
+        cudaMallocHost((void**)&m->h_ks, sizeof(KrylovScalars)) != cudaSuccess ||
+        cudaMallocHost((void**)&m->h_state, sizeof(int)) != cudaSuccess) {
         g_err = "cudaMallocHost failed"; return fail(SW2G_ERR_NOMEM);
     }
     m->M = MeshView{V, T, S, m->d_tri, m->d_ex, m->d_ey, m->d_ez, m->d_gx, m->d_gy, m->d_djac,
@@ -431,12 +447,11 @@ extern "C" void sw2g_destroy(sw2g_model* m) {
         if (m->graph64[k]) cudaGraphExecDestroy(m->graph64[k]);
         if (m->graph32[k]) cudaGraphExecDestroy(m->graph32[k]);
     }
-    if (m->gm_graph64) cudaGraphExecDestroy(m->gm_graph64);
-    if (m->gm_graph32) cudaGraphExecDestroy(m->gm_graph32);
-    if (m->gm_graph_b32) cudaGraphExecDestroy(m->gm_graph_b32);
+    m->gm_cycle64.clear(); m->gm_cycle32.clear(); m->gm_cycle_b32.clear();
     for (void* p : m->allocs) cudaFree(p);
     if (m->h_rout) cudaFreeHost(m->h_rout);
     if (m->h_ks) cudaFreeHost(m->h_ks);
+    if (m->h_state) cudaFreeHost(m->h_state);
     if (m->h_pflag) cudaFreeHost(m->h_pflag);
     if (m->h_cptr) cudaFreeHost(m->h_cptr);
     if (m->h_cown) cudaFreeHost(m->h_cown);
@@ -713,10 +728,7 @@ static void invalidate_graphs(sw2g_model* m) {
         if (m->graph64[k]) { cudaGraphExecDestroy(m->graph64[k]); m->graph64[k] = nullptr; }
         if (m->graph32[k]) { cudaGraphExecDestroy(m->graph32[k]); m->graph32[k] = nullptr; }
     }
-    if (m->gm_graph64) { cudaGraphExecDestroy(m->gm_graph64); m->gm_graph64 = nullptr; }
-    if (m->gm_graph32) { cudaGraphExecDestroy(m->gm_graph32); m->gm_graph32 = nullptr; }
-    if (m->gm_graph_b32) { cudaGraphExecDestroy(m->gm_graph_b32); m->gm_graph_b32 = nullptr; }
-    m->gm_m64 = m->gm_m32 = m->gm_mb32 = -1;
+    m->gm_cycle64.clear(); m->gm_cycle32.clear(); m->gm_cycle_b32.clear();
 }
 
 // Chunks of the flagged nodes for the AMG's level-0 corrections (amg_kernels.cu).  The
@@ -1001,51 +1013,70 @@ static bool gm_reorth() {
     return on;
 }
 
+// Captures a cycle over the given vectors (kept while the restart length stays the same)
+template <class VT>
+static int build_cycle(sw2g_model* m, CycleGraph* C, const PrecondOp<VT>& op, const VT* vals, VT* Vb, VT* z, const VT* rhs, VT* out,
+                       int mres) {
+    if (C->m == mres && C->precond == op.kind) return SW2G_OK;
+    C->clear();
+    const int n = m->n, seg = mres <= kGmSegment + 7 ? mres : kGmSegment;
+    const size_t ld = gm_ld(n);
+    for (int first = 0; first <= mres; first += seg) {   // the last round captures the end
+        const bool end = first >= mres;
+        cudaGraph_t g;
+        cudaGraphExec_t exec = nullptr;
+        CK(cudaStreamBeginCapture(m->st, cudaStreamCaptureModeThreadLocal));
+        if (end) {
+            gmres_end<VT>(m->B, op, Vb, ld, z, out, m->gm, m->st);
+        } else {
+            if (first == 0) gmres_begin<VT>(n, Vb, rhs, m->gm_rw, m->gm, m->st);
+            gmres_steps<VT>(m->B, op, vals, Vb, ld, z, m->gm_rw, m->gm, m->st, first, std::min(mres, first + seg), gm_reorth());
+        }
+        const cudaError_t e1 = cudaGetLastError();
+        const cudaError_t e2 = cudaStreamEndCapture(m->st, &g);
+        if (e1 != cudaSuccess || e2 != cudaSuccess) {
+            g_err = std::string("graph capture: ") + cudaGetErrorString(e1 != cudaSuccess ? e1 : e2);
+            C->clear();
+            return SW2G_ERR_CUDA;
+        }
+        const cudaError_t e3 = cudaGraphInstantiate(&exec, g, 0);
+        cudaGraphDestroy(g);
+        if (e3 != cudaSuccess) { C->clear(); CK(e3); }
+        if (end) C->end = exec;
+        else C->seg.push_back(exec);
+        if (!end && first + seg > mres) first = mres - seg;   // a shorter last segment: the end comes next
+    }
+    C->m = mres; C->precond = op.kind; C->per_segment = seg;
+    return SW2G_OK;
+}
+// Replays a cycle of `per_step` kernels a step; `whole`: every step, without looking at the stop flag
+static int run_cycle(sw2g_model* m, const CycleGraph& C, int per_step, bool whole) {
+    for (size_t k = 0; k < C.seg.size(); k++) {
+        if (k > 0 && !whole) {
+            CK(cudaMemcpyAsync(m->h_state, m->gm.state, sizeof(int), cudaMemcpyDeviceToHost, m->st));
+            CK(cudaStreamSynchronize(m->st));
+            if (*m->h_state) break;
+        }
+        m->prof_launch[4] += (long long)std::min(C.per_segment, C.m - (int)k * C.per_segment) * per_step;
+        CK(cudaGraphLaunch(C.seg[k], m->st));
+    }
+    CK(cudaGraphLaunch(C.end, m->st));
+    return SW2G_OK;
+}
 // FP32 cycle: FP32 basis, FP32 matrix and FP32 preconditioner on the FP32 right-hand side f_b; the
 // correction lands in f_x (the FP64 residual and the update stay with the caller)
-static int gmres_graph32(sw2g_model* m, cudaGraphExec_t* graph, int* built_m, int precond, int mres) {
-    if (*graph && *built_m == mres) return SW2G_OK;
-    if (*graph) { cudaGraphExecDestroy(*graph); *graph = nullptr; }
-    *built_m = mres;
+static int gmres_graph32(sw2g_model* m, int precond, int mres) {
     PrecondOp<float> op;
     op.kind = precond; op.right = true; op.ilu = &m->ilu; op.lu = m->f_lu; op.dinv = m->f_inv; op.amg = &m->amg;
     op.vals = m->f_vals;
-    cudaGraph_t g;
-    CK(cudaStreamBeginCapture(m->st, cudaStreamCaptureModeThreadLocal));
-    gmres_cycle<float>(m->B, op, m->f_vals, m->gm_V32, gm_ld(m->n), m->f_z, m->f_b, m->f_x, m->gm_rw, m->gm, m->st,
-                       mres, gm_reorth());
-    cudaError_t e1 = cudaGetLastError();
-    cudaError_t e2 = cudaStreamEndCapture(m->st, &g);
-    if (e1 != cudaSuccess || e2 != cudaSuccess) {
-        g_err = std::string("graph capture: ") + cudaGetErrorString(e1 != cudaSuccess ? e1 : e2);
-        return SW2G_ERR_CUDA;
-    }
-    CK(cudaGraphInstantiate(graph, g, 0));
-    cudaGraphDestroy(g);
-    return SW2G_OK;
+    return build_cycle<float>(m, &m->gm_cycle_b32, op, m->f_vals, m->gm_V32, m->f_z, m->f_b, m->f_x, mres);
 }
-
-static int gmres_graph(sw2g_model* m, cudaGraphExec_t* graph, int* built_m, bool mixed, int precond, int mres) {
-    if (*graph && *built_m == mres) return SW2G_OK;
-    if (*graph) { cudaGraphExecDestroy(*graph); *graph = nullptr; }
-    *built_m = mres;
+static int gmres_graph(sw2g_model* m, bool mixed, int precond, int mres) {
     PrecondOp<double> op;
     op.kind = precond; op.right = true; op.ilu = &m->ilu; op.lu = m->d_lu; op.dinv = m->d_inv; op.amg = &m->amg;
     op.vals = m->d_vals;
     if (mixed) { op.mixed = true; op.vals32 = m->f_vals; op.lu32 = m->f_lu; op.dinv32 = m->f_inv; op.tmp32 = m->f_z; }
-    cudaGraph_t g;
-    CK(cudaStreamBeginCapture(m->st, cudaStreamCaptureModeThreadLocal));
-    gmres_cycle<double>(m->B, op, m->d_vals, m->gm_V64, gm_ld(m->n), m->k_z, m->d_t64, m->k_xi, m->gm_rw, m->gm,
-                        m->st, mres, gm_reorth());
-    cudaError_t e1 = cudaGetLastError();
-    cudaError_t e2 = cudaStreamEndCapture(m->st, &g);
-    if (e1 != cudaSuccess || e2 != cudaSuccess) {
-        g_err = std::string("graph capture: ") + cudaGetErrorString(e1 != cudaSuccess ? e1 : e2);
-        return SW2G_ERR_CUDA;
-    }
-    CK(cudaGraphInstantiate(graph, g, 0));
-    cudaGraphDestroy(g);
-    return SW2G_OK;
+    return build_cycle<double>(m, mixed ? &m->gm_cycle32 : &m->gm_cycle64, op, m->d_vals, m->gm_V64, m->k_z, m->d_t64, m->k_xi, mres);
 }
 
 // Restarted GMRES(kGmM) on the prepared (scaled) system, FP64 Krylov basis.  Each
@@ -1087,19 +1118,18 @@ static int solve_gmres(sw2g_model* m, double* x, double* b, const sw2g_newton_op
     if (basis32) {
         if (!m->gm_V32 || m->gm_cap32 < mres) {
             TRY(gmres_basis(m, &m->gm_V32, &m->gm_cap32, mres));
-            m->gm_mb32 = -1;   // the cycle graph holds the old basis address
+            m->gm_cycle_b32.clear();   // the cycle's graphs hold the old basis address
         }
-        TRY(gmres_graph32(m, &m->gm_graph_b32, &m->gm_mb32, o.precond, mres));
+        TRY(gmres_graph32(m, o.precond, mres));
     } else {
         if (!m->gm_V64 || m->gm_cap64 < mres) {
             TRY(gmres_basis(m, &m->gm_V64, &m->gm_cap64, mres));
-            m->gm_m32 = m->gm_m64 = -1;
+            m->gm_cycle32.clear(); m->gm_cycle64.clear();
         }
-        TRY(gmres_graph(m, mixed ? &m->gm_graph32 : &m->gm_graph64, mixed ? &m->gm_m32 : &m->gm_m64, mixed, o.precond,
-                        mres));
+        TRY(gmres_graph(m, mixed, o.precond, mres));
     }
     const int pl = precond_launches(m, o.precond) + (mixed ? 2 : 0);
-    const int per_cycle = mres * (4 + pl) + 4 + pl;
+    const int per_step = 4 + pl;
     // floor: a tenth of the Newton tolerance; a hundredth under the reference's absolute test, where the
     // converged state is compared with the reference's (exact-LU) one to 1e-8 relative
     const double target = std::max(o.krylov_tol * fnorm, (o.tol_nonlin_rel > 0.0 ? 0.1 : 0.01) * o.tol_nonlin);
@@ -1158,13 +1188,13 @@ static int solve_gmres(sw2g_model* m, double* x, double* b, const sw2g_newton_op
         if (rtol < (basis32 ? 1e-5 : 1e-12)) rtol = basis32 ? 1e-5 : 1e-12;   // FP32 resolves no more per cycle
         CK(cudaMemcpyAsync(m->gm.scal + 3, &rtol, sizeof(double), cudaMemcpyHostToDevice, m->st));
         {
-            ProfScope ps(m, 4, per_cycle + 1);
+            ProfScope ps(m, 4, 5 + pl + (basis32 ? 2 : 0));   // besides the steps
             if (basis32) {   // FP32 Krylov cycle inside the FP64 refinement
                 launch_to_float(n, m->d_t64, m->f_b, m->st);
-                CK(cudaGraphLaunch(m->gm_graph_b32, m->st));
+                TRY(run_cycle(m, m->gm_cycle_b32, per_step, false));
                 launch_to_double(n, m->f_x, m->k_xi, m->st);
             } else {
-                CK(cudaGraphLaunch(mixed ? m->gm_graph32 : m->gm_graph64, m->st));
+                TRY(run_cycle(m, mixed ? m->gm_cycle32 : m->gm_cycle64, per_step, false));
             }
             launch_axpy(n, 1.0, m->k_xi, x, m->st);
             CKL();
@@ -1740,7 +1770,7 @@ extern "C" int sw2g_reset_profile(sw2g_model* m) {
 
 extern "C" int sw2g_time_kernel(sw2g_model* m, int which, int reps, double* avg_ms, double* bytes) {
     NEED(m && avg_ms && bytes && reps > 0 && which >= 0 && which <= 9, "sw2g_time_kernel: bad argument");
-    NEED(which != 8 || m->gm_graph_b32, "sw2g_time_kernel: no FP32 GMRES cycle has run yet");
+    NEED(which != 8 || m->gm_cycle_b32.m > 0, "sw2g_time_kernel: no FP32 GMRES cycle has run yet");
     const double nnz = m->nnz, n = m->n, T = m->T, S = m->S;
     if (which >= 4) {   // the AMG sweeps
         if (!m->amg_ready) TRY(build_amg(m));
@@ -1763,7 +1793,7 @@ extern "C" int sw2g_time_kernel(sw2g_model* m, int which, int reps, double* avg_
             case 7: spmv_skip<float>(m->B, m->f_vals, m->f_p, m->f_Ap, nullptr, nullptr, m->st); break;
             case 8:   // a whole FP32 GMRES cycle with its stopping test off: every iteration runs
                 cudaMemcpyAsync(m->gm.scal + 3, &zero, sizeof(double), cudaMemcpyHostToDevice, m->st);
-                cudaGraphLaunch(m->gm_graph_b32, m->st);
+                run_cycle(m, m->gm_cycle_b32, 0, true);
                 break;
             case 9: amg_patch_correct<float>(m->B, m->amg, m->f_vals, m->f_p, m->f_Ap, nullptr, m->st); break;
 
@@ -1790,7 +1820,7 @@ extern "C" int sw2g_time_kernel(sw2g_model* m, int which, int reps, double* avg_
         case 6: *bytes = 4.0 * (8.0 * nnz + 32.0 * n); break;   // ~4 level-0 matrix passes (coarse levels extra)
         case 5: *bytes = 8.0 * nnz + 12.0 * n + 12.0 * n + 8.0 * n; break;   // FP32 SpMV + FP32 block apply
         case 7: *bytes = 8.0 * nnz + 12.0 * n; break;                        // FP32 values + cols, x and y
-        case 8: *bytes = (double)m->gm_mb32; break;                          // iterations of the cycle (not bytes)
+        case 8: *bytes = (double)m->gm_cycle_b32.m; break;                          // iterations of the cycle (not bytes)
         case 9: *bytes = 4.0 * (double)m->p_rtot + 12.0 * m->p_nentries; break;   // FP32 inverse rows + residuals
     }
     return SW2G_OK;

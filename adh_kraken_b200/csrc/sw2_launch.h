@@ -247,11 +247,15 @@ struct GmresDev {                       // device buffers of one cycle
     int* state = nullptr;               // [0] done, [1] columns built, [2] status (0 ok, 1 breakdown, 2 non-finite)
     double* scal = nullptr;             // [0] beta, [1] target, [2] residual estimate, [3] rtol (host-set), [4] h_{j+1,j}
 };
-// out = M^-1 V_k y from one cycle on rhs (x0 = 0), minimising the rw-weighted
-// residual 2-norm; Vb holds kGmM+1 vectors of stride ld
+// One cycle, out = M^-1 V_k y on rhs (x0 = 0), minimising the rw-weighted residual 2-norm: begin, steps 0 .. m-1 (steps
+// after convergence do nothing), end.  Vb holds m+1 vectors of stride ld; z is a work vector.
 template <class VT>
-void gmres_cycle(const BlockCSR& A, const PrecondOp<VT>& P, const VT* vals, VT* Vb, size_t ld, VT* z, const VT* rhs,
-                 VT* out, const double* rw, const GmresDev& G, cudaStream_t st, int m, bool reorth);
+void gmres_begin(int n, VT* Vb, const VT* rhs, const double* rw, const GmresDev& G, cudaStream_t st);
+template <class VT>
+void gmres_steps(const BlockCSR& A, const PrecondOp<VT>& P, const VT* vals, VT* Vb, size_t ld, VT* z, const double* rw,
+                 const GmresDev& G, cudaStream_t st, int first, int last, bool reorth);
+template <class VT>
+void gmres_end(const BlockCSR& A, const PrecondOp<VT>& P, VT* Vb, size_t ld, VT* z, VT* out, const GmresDev& G, cudaStream_t st);
 // rw_i = 1 / s_i (weights that make a scaled system's residual the unscaled one)
 void launch_inv_scale(int n, const double* scale, double* rw, cudaStream_t st);
 template <class VT>
