@@ -411,6 +411,7 @@ extern "C" int sw2g_create(const sw2g_mesh* mesh, void* cuda_stream, sw2g_model*
         return fail(rc);
     CK(cudaMemsetAsync(m->d_counter, 0, sizeof(unsigned int), m->st));
     CK(cudaMemsetAsync(m->d_bc_mask, 0, sizeof(int) * n, m->st));
+    CK(cudaMemsetAsync(m->d_wd, 0, sizeof(int) * (size_t)T, m->st));
     CK(cudaMemsetAsync(m->d_dirichlet, 0, sizeof(double) * n, m->st));
     CK(cudaMemsetAsync(m->d_EJ, 0, sizeof(double) * 81 * (size_t)m->Etot, m->st));
     CK(cudaMemsetAsync(m->d_ER, 0, sizeof(double) * 9 * (size_t)m->Etot, m->st));
@@ -510,17 +511,19 @@ static int do_wd(sw2g_model* m, const double* sol, const double* sol_old) {
     CKL();
     return SW2G_OK;
 }
-static int do_residual(sw2g_model* m, const double* sol, const double* sol_old, const double* sol_older, double* res) {
-    ProfScope ps(m, 0, 3);
-    launch_elem_resid(m->M, m->P, sol, sol_old, sol_older, m->d_wd, m->d_ER, m->st);
+// wd: wet/dry flags of the Newton solve's start, or null for those of the states given (the element kernels then
+// derive the one they look at, so no flag pass runs)
+static int do_residual(sw2g_model* m, const double* sol, const double* sol_old, const double* sol_older, const int* wd, double* res) {
+    ProfScope ps(m, 0, 2);
+    launch_elem_resid(m->M, m->P, sol, sol_old, sol_older, wd, m->d_ER, m->st);
     launch_gather_resid(m->V, m->A, m->d_ER, res, m->st);
     CKL();
     return SW2G_OK;
 }
-static int do_jacobian(sw2g_model* m, const double* sol, const double* sol_old, const double* sol_older, double* vals) {
+static int do_jacobian(sw2g_model* m, const double* sol, const double* sol_old, const double* sol_older, const int* wd, double* vals) {
     {
         ProfScope ps(m, 1, 4);
-        launch_elem_jac(m->M, m->P, sol, sol_old, sol_older, m->d_wd, m->d_EJ, m->st);
+        launch_elem_jac(m->M, m->P, sol, sol_old, sol_older, wd, m->d_EJ, m->st);
         CKL();
     }
     ProfScope ps(m, 2, 1);
@@ -1351,7 +1354,7 @@ static int newton_device(sw2g_model* m, const sw2g_newton_opts& o_in, sw2g_newto
     }
     CK(cudaMemsetAsync(m->d_dsol, 0, sizeof(double) * n, m->st));
     double rmax, rl2, imax;
-    TRY(do_residual(m, m->d_sol, m->d_sol_old, m->d_sol_older, m->d_res));
+    TRY(do_residual(m, m->d_sol, m->d_sol_old, m->d_sol_older, m->d_wd, m->d_res));
     TRY(do_norms(m, m->d_res, m->d_dsol, &rmax, &rl2, &imax));
     if (!std::isfinite(rl2)) { g_err = "non-finite residual at the initial guess"; return SW2G_ERR_NONFINITE; }
     st.prev_resid_max = rmax;
@@ -1367,7 +1370,7 @@ static int newton_device(sw2g_model* m, const sw2g_newton_opts& o_in, sw2g_newto
             CKL();
         }
         double gmax, gl2, gi;
-        TRY(do_residual(m, m->d_sol, m->d_sol_old, m->d_sol_older, m->d_res));
+        TRY(do_residual(m, m->d_sol, m->d_sol_old, m->d_sol_older, m->d_wd, m->d_res));
         TRY(do_norms(m, m->d_res, m->d_dsol, &gmax, &gl2, &gi));
         static const bool trace = getenv("SW2G_TRACE_NEWTON") != nullptr;
         if (trace)
@@ -1382,7 +1385,7 @@ static int newton_device(sw2g_model* m, const sw2g_newton_opts& o_in, sw2g_newto
                 launch_masked_copy(n, m->d_bc_mask, m->d_dirichlet, m->d_sol, m->st);
                 CKL();
             }
-            TRY(do_residual(m, m->d_sol, m->d_sol_old, m->d_sol_older, m->d_res));
+            TRY(do_residual(m, m->d_sol, m->d_sol_old, m->d_sol_older, m->d_wd, m->d_res));
             TRY(do_norms(m, m->d_res, m->d_dsol, &rmax, &rl2, &imax));
         }
     }
@@ -1394,7 +1397,7 @@ static int newton_device(sw2g_model* m, const sw2g_newton_opts& o_in, sw2g_newto
     int it = 0, stalled_its = 0; bool ok = true, keep, lin_ok = true;
     double rmax_prev = rmax;
     do {
-        TRY(do_jacobian(m, m->d_sol, m->d_sol_old, m->d_sol_older, m->d_vals));
+        TRY(do_jacobian(m, m->d_sol, m->d_sol_old, m->d_sol_older, m->d_wd, m->d_vals));
         CK(cudaMemsetAsync(m->d_dsol, 0, sizeof(double) * n, m->st));
         TRY(do_prepare(m, m->d_vals, m->d_res, m->d_dsol));
         TRY(do_precond_setup(m, m->d_vals, o.precond, o.amg_chunks));
@@ -1415,7 +1418,7 @@ static int newton_device(sw2g_model* m, const sw2g_newton_opts& o_in, sw2g_newto
             CKL();
         }
         const double old_l2 = rl2;
-        TRY(do_residual(m, m->d_sol, m->d_sol_old, m->d_sol_older, m->d_res));
+        TRY(do_residual(m, m->d_sol, m->d_sol_old, m->d_sol_older, m->d_wd, m->d_res));
         TRY(do_norms(m, m->d_res, m->d_dsol, &rmax, &rl2, &imax));
         int cuts = 0;   // line search, fe_newton.c:681-741
         // a step into a state whose residual is not finite is cut like a step that raised the residual
@@ -1427,7 +1430,7 @@ static int newton_device(sw2g_model* m, const sw2g_newton_opts& o_in, sw2g_newto
                 launch_axpy(n, 1.0, m->d_dsol, m->d_sol, m->st);
                 CKL();
             }
-            TRY(do_residual(m, m->d_sol, m->d_sol_old, m->d_sol_older, m->d_res));
+            TRY(do_residual(m, m->d_sol, m->d_sol_old, m->d_sol_older, m->d_wd, m->d_res));
             TRY(do_norms(m, m->d_res, m->d_dsol, &rmax, &rl2, &imax));
             cuts++;
         }
@@ -1495,10 +1498,9 @@ extern "C" int sw2g_elem_resid(sw2g_model* m, const double* sol, const double* s
                                double* out_tri, double* out_seg) {
     NEED(m && sol && sol_old && sol_older && out_tri && (m->S == 0 || out_seg), "sw2g_elem_resid: null argument");
     TRY(put3(m, sol, sol_old, sol_older));
-    TRY(do_wd(m, m->d_sol, m->d_sol_old));
     {
-        ProfScope ps(m, 0, 2);
-        launch_elem_resid(m->M, m->P, m->d_sol, m->d_sol_old, m->d_sol_older, m->d_wd, m->d_ER, m->st);
+        ProfScope ps(m, 0, 1);
+        launch_elem_resid(m->M, m->P, m->d_sol, m->d_sol_old, m->d_sol_older, nullptr, m->d_ER, m->st);
         CKL();
     }
     std::vector<double> er(9 * (size_t)m->Etot);
@@ -1513,10 +1515,9 @@ extern "C" int sw2g_elem_jac(sw2g_model* m, const double* sol, const double* sol
                              double* out_tri, double* out_seg) {
     NEED(m && sol && sol_old && sol_older && out_tri && (m->S == 0 || out_seg), "sw2g_elem_jac: null argument");
     TRY(put3(m, sol, sol_old, sol_older));
-    TRY(do_wd(m, m->d_sol, m->d_sol_old));
     {
         ProfScope ps(m, 1, 4);
-        launch_elem_jac(m->M, m->P, m->d_sol, m->d_sol_old, m->d_sol_older, m->d_wd, m->d_EJ, m->st);
+        launch_elem_jac(m->M, m->P, m->d_sol, m->d_sol_old, m->d_sol_older, nullptr, m->d_EJ, m->st);
         CKL();
     }
     std::vector<double> ej(81 * (size_t)m->Etot);
@@ -1534,8 +1535,7 @@ extern "C" int sw2g_assemble_residual(sw2g_model* m, const double* sol, const do
                                       double* residual) {
     NEED(m && sol && sol_old && sol_older && residual, "sw2g_assemble_residual: null argument");
     TRY(put3(m, sol, sol_old, sol_older));
-    TRY(do_wd(m, m->d_sol, m->d_sol_old));
-    TRY(do_residual(m, m->d_sol, m->d_sol_old, m->d_sol_older, m->d_res));
+    TRY(do_residual(m, m->d_sol, m->d_sol_old, m->d_sol_older, nullptr, m->d_res));
     CK(cudaMemcpyAsync(residual, m->d_res, sizeof(double) * m->n, cudaMemcpyDeviceToHost, m->st));
     CK(cudaStreamSynchronize(m->st));
     return SW2G_OK;
@@ -1545,8 +1545,7 @@ extern "C" int sw2g_assemble_jacobian(sw2g_model* m, const double* sol, const do
                                       double* vals) {
     NEED(m && sol && sol_old && sol_older && vals, "sw2g_assemble_jacobian: null argument");
     TRY(put3(m, sol, sol_old, sol_older));
-    TRY(do_wd(m, m->d_sol, m->d_sol_old));
-    TRY(do_jacobian(m, m->d_sol, m->d_sol_old, m->d_sol_older, m->d_vals));
+    TRY(do_jacobian(m, m->d_sol, m->d_sol_old, m->d_sol_older, nullptr, m->d_vals));
     CK(cudaMemcpyAsync(vals, m->d_vals, sizeof(double) * m->nnz, cudaMemcpyDeviceToHost, m->st));
     CK(cudaStreamSynchronize(m->st));
     return SW2G_OK;
@@ -1568,7 +1567,7 @@ extern "C" int sw2g_assemble_residual_wd(sw2g_model* m, const double* sol, const
     NEED(m && sol && sol_old && sol_older && wd_flag && residual, "sw2g_assemble_residual_wd: null argument");
     TRY(put_wd(m, wd_flag));
     TRY(put3(m, sol, sol_old, sol_older));
-    TRY(do_residual(m, m->d_sol, m->d_sol_old, m->d_sol_older, m->d_res));
+    TRY(do_residual(m, m->d_sol, m->d_sol_old, m->d_sol_older, m->d_wd, m->d_res));
     CK(cudaMemcpyAsync(residual, m->d_res, sizeof(double) * m->n, cudaMemcpyDeviceToHost, m->st));
     CK(cudaStreamSynchronize(m->st));
     return SW2G_OK;
@@ -1579,7 +1578,7 @@ extern "C" int sw2g_assemble_jacobian_wd(sw2g_model* m, const double* sol, const
     NEED(m && sol && sol_old && sol_older && wd_flag && vals, "sw2g_assemble_jacobian_wd: null argument");
     TRY(put_wd(m, wd_flag));
     TRY(put3(m, sol, sol_old, sol_older));
-    TRY(do_jacobian(m, m->d_sol, m->d_sol_old, m->d_sol_older, m->d_vals));
+    TRY(do_jacobian(m, m->d_sol, m->d_sol_old, m->d_sol_older, m->d_wd, m->d_vals));
     CK(cudaMemcpyAsync(vals, m->d_vals, sizeof(double) * m->nnz, cudaMemcpyDeviceToHost, m->st));
     CK(cudaStreamSynchronize(m->st));
     return SW2G_OK;
@@ -1830,19 +1829,17 @@ extern "C" int sw2g_time_kernel(sw2g_model* m, int which, int reps, double* avg_
 // For callers that cannot allocate device memory when they call in: an application
 // that hands all free device memory to its own pool at start-up, or a time loop
 // that must not allocate (or free) inside its steps.  sw2g_assemble_residual keeps
-// its element-residual and wet/dry work buffers in memory that sw2g_create
-// allocated; this variant keeps them in file-scope device arrays of a fixed size
-// instead, so a call allocates nothing.  Every GPU that loads the library holds
-// these arrays (about 10.5 MB) until the process exits.
+// its element-residual work buffer in memory that sw2g_create allocated; this
+// variant keeps it in a file-scope device array of a fixed size instead, so a
+// call allocates nothing.  Every GPU that loads the library holds this array
+// (about 9.5 MB) until the process exits.
 constexpr int kNoAllocMaxElems = 1 << 17;   // triangles + boundary segments
 constexpr int kNoAllocMaxNodes = 1 << 17;
 constexpr int kNoAllocMaxDevices = 64;
 static __device__ __align__(256) double g_na_elem_resid[9 * (size_t)kNoAllocMaxElems];
-static __device__ __align__(256) int g_na_wd_flags[kNoAllocMaxElems];
-static __device__ __align__(256) int g_na_node_work[kNoAllocMaxNodes];
-// device addresses of the arrays, looked up once per device (host code may not use
-// the arrays' names as addresses: those are host-side stand-ins)
-struct NoAllocScratch { double* er; int* wd; int* node; };
+// the array's device address, looked up once per device (host code may not use the array's
+// name as an address: that is a host-side stand-in)
+struct NoAllocScratch { double* er; };
 static NoAllocScratch g_na_ptr[kNoAllocMaxDevices];
 static bool g_na_ready[kNoAllocMaxDevices];
 static std::mutex g_na_mutex;
@@ -1861,8 +1858,6 @@ static int noalloc_scratch(const sw2g_model* m, NoAllocScratch* out) {
     if (!g_na_ready[dev]) {
         NoAllocScratch p{};
         CK(cudaGetSymbolAddress((void**)&p.er, g_na_elem_resid));
-        CK(cudaGetSymbolAddress((void**)&p.wd, g_na_wd_flags));
-        CK(cudaGetSymbolAddress((void**)&p.node, g_na_node_work));
         g_na_ptr[dev] = p;
         g_na_ready[dev] = true;
     }
@@ -1880,11 +1875,9 @@ extern "C" int sw2g_assemble_residual_noalloc(sw2g_model* m, const double* d_sol
     }
     NoAllocScratch S{};
     TRY(noalloc_scratch(m, &S));
-    // every entry of the three arrays that the gather reads is written first by this call
-    // (wet/dry node marks, element flags, 9 (6) residual entries per triangle (segment)), so
-    // nothing needs clearing between calls
-    launch_wd_flags(m->M, d_sol, d_sol_old, S.node, S.wd, m->st);
-    launch_elem_resid(m->M, m->P, d_sol, d_sol_old, d_sol_older, S.wd, S.er, m->st);
+    // every entry of the array that the gather reads is written first by this call (9 (6) residual
+    // entries per triangle (segment)), so nothing needs clearing between calls
+    launch_elem_resid(m->M, m->P, d_sol, d_sol_old, d_sol_older, nullptr, S.er, m->st);
     launch_gather_resid(m->V, m->A, S.er, d_residual, m->st);
     CKL();
     CK(cudaStreamSynchronize(m->st));

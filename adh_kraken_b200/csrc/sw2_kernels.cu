@@ -36,8 +36,26 @@ __device__ __forceinline__ void load_tri(const MeshView& M, const double* __rest
         T.hoo[a] = sol_older[3 * n]; T.veloo[a].x = sol_older[3 * n + 1]; T.veloo[a].y = sol_older[3 * n + 2];
     }
     T.djac = M.djac[e];
-    T.wd_flag = wd_flag[e];
+    // without flags of an earlier state: the only one the residual looks at, dry at both levels (fe_sw2_wdflag_legacy)
+    T.wd_flag = wd_flag ? wd_flag[e]
+                        : (T.h[0] < 0 && T.h[1] < 0 && T.h[2] < 0 && T.ho[0] < 0 && T.ho[1] < 0 && T.ho[2] < 0) ? 2 : 0;
 }
+// every depth positive, at the current level by more than `margin`
+__device__ __forceinline__ bool all_wet(const TriData& T, double margin) {
+    bool w = true;
+#pragma unroll
+    for (int a = 0; a < 3; a++) w = w && T.h[a] > margin && T.ho[a] > 0.0 && T.hoo[a] > 0.0;
+    return w;
+}
+// What bounds the element kernels is latency: 1600 instructions a residual, most of them FP64 in long chains (13
+// divisions, 6 square roots), at few warps an SM.  Elements that are wet at all levels, most of them, take a
+// branch without the cut sub-triangles' code (~1000 operations left), and kElemBlocks CTAs an SM, 168 registers,
+// is the best of 2 to 5 for the two branches together (FD Jacobian of 1M wet triangles: 1.43, 1.29, 1.49, 1.75 ms; 2.42 ms
+// with the general code for all, at 254 registers).  Kernels of their own for the wet and the cut elements pay the loads
+// twice (1.80 ms).
+// Neighbouring elements stay in neighbouring blocks: spreading the cut ones over the grid mixes the two branches' code in
+// every SM's instruction cache (FD Jacobian of a 250k-triangle beach 0.64 -> 0.87 ms).
+constexpr int kElemThreads = 128, kElemBlocks = 3;
 
 __device__ __forceinline__ SegBC seg_bc(const StepParams& P) {
     return SegBC{P.bc_depth, P.bc_vx, P.bc_vy, P.bc_qs, P.bc_convey, P.bc_rough, P.bc_tail, P.bc_flux};
@@ -85,23 +103,31 @@ __global__ void k_dry_mask(int nnodes, const double* __restrict__ sol_old, int* 
 }
 
 // ---------------------------------------------------------------- residuals
-__global__ void __launch_bounds__(128) k_resid_tri(MeshView M, StepParams P, const double* __restrict__ sol,
+__device__ __forceinline__ void seg_residual(const MeshView& M, const StepParams& P, const double* __restrict__ sol, int s,
+                                             double* __restrict__ ER);
+// triangles, and after their blocks the boundary segments
+__global__ void __launch_bounds__(kElemThreads, kElemBlocks) k_resid(MeshView M, StepParams P, int tri_blocks, const double* __restrict__ sol,
                                                    const double* __restrict__ sol_old, const double* __restrict__ sol_older,
                                                    const int* __restrict__ wd_flag, double* __restrict__ ER) {
-    int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if ((int)blockIdx.x >= tri_blocks) {
+        const int s = (blockIdx.x - tri_blocks) * blockDim.x + threadIdx.x;
+        if (s < M.nseg) seg_residual(M, P, sol, s, ER);
+        return;
+    }
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= M.ntri) return;
     TriData T;
     load_tri(M, sol, sol_old, sol_older, wd_flag, e, T);
     double r[9];
-    body_resid<true>(T, P.dt, P.alpha, P.grav, r);
+    if (all_wet(T, 0.0)) body_resid<true, true>(T, P.dt, P.alpha, P.grav, r);
+    else body_resid<true, false>(T, P.dt, P.alpha, P.grav, r);
     double* out = ER + 9 * (size_t)e;
 #pragma unroll
     for (int i = 0; i < 9; i++) out[i] = r[i];
 }
 
-__global__ void k_resid_seg(MeshView M, StepParams P, const double* __restrict__ sol, double* __restrict__ ER) {
-    int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= M.nseg) return;
+__device__ __forceinline__ void seg_residual(const MeshView& M, const StepParams& P, const double* __restrict__ sol, int s,
+                                             double* __restrict__ ER) {
     SegData S;
     load_seg(M, sol, s, S);
     double r[6];
@@ -132,15 +158,8 @@ __global__ void k_gather_resid(int nnodes, AssemblyMaps A, const double* __restr
 // column (node i, var k) = (R(u + eps e) - R(u - eps e)) / (2 eps).
 // Template VAR: 0 perturbs h (pressure terms evaluated), 1/2 perturb u/v
 // (pressure terms skipped, as the reference's PRESSURE_FLAG does).
-template <int VAR>
-__global__ void __launch_bounds__(128) k_fd_tri(MeshView M, StepParams P, const double* __restrict__ sol,
-                                                const double* __restrict__ sol_old, const double* __restrict__ sol_older,
-                                                const int* __restrict__ wd_flag, double* __restrict__ EJ, int Etot) {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    const int i = blockIdx.y;          // perturbed node 0..2
-    if (e >= M.ntri) return;
-    TriData T;
-    load_tri(M, sol, sol_old, sol_older, wd_flag, e, T);
+template <int VAR, bool WET>
+__device__ __forceinline__ void fd_column(const TriData& T, const StepParams& P, int i, double* __restrict__ out) {
     double u0 = VAR == 0 ? (i == 0 ? T.h[0] : i == 1 ? T.h[1] : T.h[2])
               : VAR == 1 ? (i == 0 ? T.vel[0].x : i == 1 ? T.vel[1].x : T.vel[2].x)
                          : (i == 0 ? T.vel[0].y : i == 1 ? T.vel[1].y : T.vel[2].y);
@@ -158,12 +177,24 @@ __global__ void __launch_bounds__(128) k_fd_tri(MeshView M, StepParams P, const 
             else if (VAR == 1) Q.vel[a].x += d;
             else Q.vel[a].y += d;
         }
-        body_resid<VAR == 0>(Q, P.dt, P.alpha, P.grav, sgn == 0 ? Rp : Rm);
+        body_resid<VAR == 0, WET>(Q, P.dt, P.alpha, P.grav, sgn == 0 ? Rp : Rm);
     }
-    const int col = i * 3 + VAR;
-    double* out = EJ + ((size_t)col * Etot + e) * 9;
 #pragma unroll
     for (int r = 0; r < 9; r++) out[r] = (Rp[r] - Rm[r]) / eps2;
+}
+template <int VAR>
+__global__ void __launch_bounds__(kElemThreads, kElemBlocks) k_fd_tri(MeshView M, StepParams P, const double* __restrict__ sol,
+                                                const double* __restrict__ sol_old, const double* __restrict__ sol_older,
+                                                const int* __restrict__ wd_flag, double* __restrict__ EJ, int Etot) {
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = blockIdx.y;          // perturbed node 0..2
+    if (e >= M.ntri) return;
+    TriData T;
+    load_tri(M, sol, sol_old, sol_older, wd_flag, e, T);
+    double* out = EJ + ((size_t)(i * 3 + VAR) * Etot + e) * 9;
+    // a depth above 2e-4 stays positive under its perturbation (fd_eps: at most 1e-4, or 1e-4 of it)
+    if (all_wet(T, VAR == 0 ? 2e-4 : 0.0)) fd_column<VAR, true>(T, P, i, out);
+    else fd_column<VAR, false>(T, P, i, out);
 }
 
 __global__ void k_fd_seg(MeshView M, StepParams P, const double* __restrict__ sol, double* __restrict__ EJ, int Etot) {
@@ -346,8 +377,8 @@ void launch_dry_mask(int nnodes, const double* sol_old, int* bc_mask, cudaStream
 
 void launch_elem_resid(const MeshView& M, const StepParams& P, const double* sol, const double* sol_old,
                        const double* sol_older, const int* wd_flag, double* ER, cudaStream_t st) {
-    if (M.ntri) k_resid_tri<<<blocks(M.ntri, 128), 128, 0, st>>>(M, P, sol, sol_old, sol_older, wd_flag, ER);
-    if (M.nseg) k_resid_seg<<<blocks(M.nseg, 128), 128, 0, st>>>(M, P, sol, ER);
+    const int nt = blocks(M.ntri, kElemThreads);
+    k_resid<<<nt + blocks(M.nseg, kElemThreads), kElemThreads, 0, st>>>(M, P, nt, sol, sol_old, sol_older, wd_flag, ER);
 }
 
 void launch_gather_resid(int nnodes, const AssemblyMaps& A, const double* ER, double* residual, cudaStream_t st) {
@@ -358,10 +389,10 @@ void launch_elem_jac(const MeshView& M, const StepParams& P, const double* sol, 
                      const double* sol_older, const int* wd_flag, double* EJ, cudaStream_t st) {
     const int Etot = M.ntri + M.nseg;
     if (M.ntri) {
-        dim3 g(blocks(M.ntri, 128), 3);
-        k_fd_tri<0><<<g, 128, 0, st>>>(M, P, sol, sol_old, sol_older, wd_flag, EJ, Etot);
-        k_fd_tri<1><<<g, 128, 0, st>>>(M, P, sol, sol_old, sol_older, wd_flag, EJ, Etot);
-        k_fd_tri<2><<<g, 128, 0, st>>>(M, P, sol, sol_old, sol_older, wd_flag, EJ, Etot);
+        dim3 g(blocks(M.ntri, kElemThreads), 3);
+        k_fd_tri<0><<<g, kElemThreads, 0, st>>>(M, P, sol, sol_old, sol_older, wd_flag, EJ, Etot);
+        k_fd_tri<1><<<g, kElemThreads, 0, st>>>(M, P, sol, sol_old, sol_older, wd_flag, EJ, Etot);
+        k_fd_tri<2><<<g, kElemThreads, 0, st>>>(M, P, sol, sol_old, sol_older, wd_flag, EJ, Etot);
     }
     if (M.nseg) {
         dim3 g(blocks(M.nseg, 128), 6);

@@ -9,6 +9,7 @@ namespace sw2 {
 void launch_wd_flags(const MeshView& M, const double* sol, const double* sol_old, int* node_tmp, int* wd_flag,
                      cudaStream_t st);
 void launch_dry_mask(int nnodes, const double* sol_old, int* bc_mask, cudaStream_t st);
+// wd_flag: flags of an earlier state, or null for those of (sol, sol_old)
 void launch_elem_resid(const MeshView& M, const StepParams& P, const double* sol, const double* sol_old,
                        const double* sol_older, const int* wd_flag, double* ER, cudaStream_t st);
 void launch_gather_resid(int nnodes, const AssemblyMaps& A, const double* ER, double* residual, cudaStream_t st);

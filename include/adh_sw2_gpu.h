@@ -210,7 +210,7 @@ int sw2g_grid_mass(sw2g_model *m, const double *sol, double density, double dt, 
  * allocate device memory when they call in (an application that gave all free device
  * memory to its own pool at start-up, a time loop that must not allocate inside its
  * steps).  No counterpart in the reference.  The call allocates nothing: its work
- * arrays are fixed-size device arrays inside the library (about 10.5 MB, held by every
+ * array is a fixed-size device array inside the library (about 9.5 MB, held by every
  * GPU that loads it until the process exits), so the mesh may have at most 131072
  * elements (triangles + segments) and 131072 nodes; larger meshes get SW2G_ERR_ARG.
  * d_sol, d_sol_old, d_sol_older [ndofs] and d_residual [ndofs] are device pointers on
