@@ -10,7 +10,9 @@
 #include <cstdlib>
 #include <cstring>
 #include <cmath>
+#include <condition_variable>
 #include <mutex>
+#include <thread>
 #include <vector>
 #include <algorithm>
 #include <string>
@@ -95,6 +97,8 @@ struct sw2g_model {
     double *d_partial = nullptr, *d_rout = nullptr; unsigned int* d_counter = nullptr;
     KrylovScalars* d_ks = nullptr;
     double* h_rout = nullptr; KrylovScalars* h_ks = nullptr; int* h_state = nullptr;   // pinned
+    char* h_stage = nullptr;           // pinned ring of large downloads (models whose matrix is one), kStageSlots pieces
+    std::vector<cudaEvent_t> stage_ev;
     cudaGraphExec_t graph64[3] = {nullptr, nullptr, nullptr}, graph32[3] = {nullptr, nullptr, nullptr};   // [precond]
     // multicolour block ILU(0)
     std::vector<int> h_color_ptr;
@@ -151,6 +155,89 @@ template <class T>
 static int upload(sw2g_model* m, T** p, const T* h, size_t count) {
     TRY(dalloc(m, p, count));
     if (count) CK(cudaMemcpyAsync(*p, h, sizeof(T) * count, cudaMemcpyHostToDevice, m->st));
+    return SW2G_OK;
+}
+
+// ------------------------------------------------------------------ large downloads
+// Device to host for results of kStageMin bytes and more.  A copy into pageable memory runs at 5 GB/s here (the driver's
+// single thread also takes the page faults of a fresh array): 12.7 of the 14.9 ms of assemble_jacobian at 250k
+// triangles.  Pieces go to a pinned ring instead, from where a few threads copy them on, so that PCIe, the copies and
+// the page faults of several cores overlap.  The threads live for the call; without them (or without the ring) the plain
+// copy is made.  Destinations that are pinned already are copied to directly.  Complete on return.
+static const size_t kStageMin = 8u << 20, kStagePiece = 1u << 20;
+static const int kStageSlots = 16, kStageThreads = 8;
+static int download(sw2g_model* m, void* dst, const void* src, size_t bytes) {
+    cudaPointerAttributes at{};
+    bool plain = bytes < kStageMin || !m->h_stage;
+    if (!plain) {
+        if (cudaPointerGetAttributes(&at, dst) != cudaSuccess) cudaGetLastError();
+        else plain = at.type != cudaMemoryTypeUnregistered;
+    }
+    const unsigned cores = std::thread::hardware_concurrency();
+    const int nt = (int)std::min<unsigned>(kStageThreads, cores ? cores : 1);
+    if (plain || nt < 2) {
+        CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, m->st));
+        CK(cudaStreamSynchronize(m->st));
+        return SW2G_OK;
+    }
+    const long pieces = (long)((bytes + kStagePiece - 1) / kStagePiece);
+    std::mutex mu;
+    std::condition_variable cv;
+    long issued = 0;                       // pieces whose copy to the ring is in the stream
+    std::vector<char> done(pieces, 0);     // pieces copied on
+    cudaError_t err = cudaSuccess;         // the first failure; everyone stops
+    auto work = [&](int w) {
+        cudaSetDevice(m->device);
+        for (long k = w; k < pieces; k += nt) {
+            {
+                std::unique_lock<std::mutex> lock(mu);
+                cv.wait(lock, [&] { return issued > k || err != cudaSuccess; });
+                if (err != cudaSuccess) return;
+            }
+            const int slot = (int)(k % kStageSlots);
+            const cudaError_t e = cudaEventSynchronize(m->stage_ev[slot]);
+            if (e == cudaSuccess)
+                memcpy((char*)dst + k * kStagePiece, m->h_stage + slot * kStagePiece, std::min(kStagePiece, bytes - k * kStagePiece));
+            std::lock_guard<std::mutex> lock(mu);
+            if (e != cudaSuccess && err == cudaSuccess) err = e;
+            done[k] = 1;
+            cv.notify_all();
+        }
+    };
+    std::vector<std::thread> team;
+    try {
+        team.reserve(nt);
+        for (int w = 0; w < nt; w++) team.emplace_back(work, w);
+    } catch (...) {   // no (more) threads: stop those that started and copy plainly
+        {
+            std::lock_guard<std::mutex> lock(mu);
+            err = cudaErrorUnknown;
+            cv.notify_all();
+        }
+        for (std::thread& t : team) t.join();
+        CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, m->st));
+        CK(cudaStreamSynchronize(m->st));
+        return SW2G_OK;
+    }
+    for (long k = 0; k < pieces; k++) {
+        if (k >= kStageSlots) {            // the slot's last piece has left it
+            std::unique_lock<std::mutex> lock(mu);
+            cv.wait(lock, [&] { return done[k - kStageSlots] || err != cudaSuccess; });
+            if (err != cudaSuccess) break;
+        }
+        const int slot = (int)(k % kStageSlots);
+        cudaError_t e = cudaMemcpyAsync(m->h_stage + slot * kStagePiece, (const char*)src + k * kStagePiece,
+                                        std::min(kStagePiece, bytes - k * kStagePiece), cudaMemcpyDeviceToHost, m->st);
+        if (e == cudaSuccess) e = cudaEventRecord(m->stage_ev[slot], m->st);
+        std::lock_guard<std::mutex> lock(mu);
+        if (e != cudaSuccess && err == cudaSuccess) err = e;
+        issued = k + 1;
+        cv.notify_all();
+        if (err != cudaSuccess) break;
+    }
+    for (std::thread& t : team) t.join();
+    CK(err);
+    CK(cudaStreamSynchronize(m->st));
     return SW2G_OK;
 }
 
@@ -420,6 +507,16 @@ extern "C" int sw2g_create(const sw2g_mesh* mesh, void* cuda_stream, sw2g_model*
         cudaMallocHost((void**)&m->h_state, sizeof(int)) != cudaSuccess) {
         g_err = "cudaMallocHost failed"; return fail(SW2G_ERR_NOMEM);
     }
+    if (sizeof(double) * (size_t)m->nnz >= kStageMin) {   // without the ring large downloads are plain copies
+        if (cudaMallocHost((void**)&m->h_stage, kStageSlots * kStagePiece) != cudaSuccess) { cudaGetLastError(); m->h_stage = nullptr; }
+        for (int k = 0; m->h_stage && k < kStageSlots; k++) {
+            cudaEvent_t e;
+            if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess) { m->stage_ev.push_back(e); continue; }
+            cudaGetLastError();
+            cudaFreeHost(m->h_stage);
+            m->h_stage = nullptr;
+        }
+    }
     m->M = MeshView{V, T, S, m->d_tri, m->d_ex, m->d_ey, m->d_ez, m->d_gx, m->d_gy, m->d_djac,
                     m->d_seg, m->d_snx, m->d_sny, m->d_sdjac, m->d_skind, m->d_sz0};
     m->A = AssemblyMaps{m->nslots, m->d_rptr, m->d_rmap, m->d_jptr, m->d_jmap, m->d_boff, m->d_blen};
@@ -453,6 +550,8 @@ extern "C" void sw2g_destroy(sw2g_model* m) {
     if (m->h_rout) cudaFreeHost(m->h_rout);
     if (m->h_ks) cudaFreeHost(m->h_ks);
     if (m->h_state) cudaFreeHost(m->h_state);
+    if (m->h_stage) cudaFreeHost(m->h_stage);
+    for (cudaEvent_t e : m->stage_ev) cudaEventDestroy(e);
     if (m->h_pflag) cudaFreeHost(m->h_pflag);
     if (m->h_cptr) cudaFreeHost(m->h_cptr);
     if (m->h_cown) cudaFreeHost(m->h_cown);
@@ -1546,9 +1645,7 @@ extern "C" int sw2g_assemble_jacobian(sw2g_model* m, const double* sol, const do
     NEED(m && sol && sol_old && sol_older && vals, "sw2g_assemble_jacobian: null argument");
     TRY(put3(m, sol, sol_old, sol_older));
     TRY(do_jacobian(m, m->d_sol, m->d_sol_old, m->d_sol_older, nullptr, m->d_vals));
-    CK(cudaMemcpyAsync(vals, m->d_vals, sizeof(double) * m->nnz, cudaMemcpyDeviceToHost, m->st));
-    CK(cudaStreamSynchronize(m->st));
-    return SW2G_OK;
+    return download(m, vals, m->d_vals, sizeof(double) * (size_t)m->nnz);
 }
 
 // The same two assemblies with the caller's wet/dry flags: inside fe_newton the
@@ -1579,9 +1676,7 @@ extern "C" int sw2g_assemble_jacobian_wd(sw2g_model* m, const double* sol, const
     TRY(put_wd(m, wd_flag));
     TRY(put3(m, sol, sol_old, sol_older));
     TRY(do_jacobian(m, m->d_sol, m->d_sol_old, m->d_sol_older, m->d_wd, m->d_vals));
-    CK(cudaMemcpyAsync(vals, m->d_vals, sizeof(double) * m->nnz, cudaMemcpyDeviceToHost, m->st));
-    CK(cudaStreamSynchronize(m->st));
-    return SW2G_OK;
+    return download(m, vals, m->d_vals, sizeof(double) * (size_t)m->nnz);
 }
 
 extern "C" int sw2g_prepare_system(sw2g_model* m, double* vals, double* residual, double* x, int* bc_mask, double* scale) {
@@ -1592,7 +1687,7 @@ extern "C" int sw2g_prepare_system(sw2g_model* m, double* vals, double* residual
     CK(cudaMemcpyAsync(m->d_dsol, x, sizeof(double) * n, cudaMemcpyHostToDevice, m->st));
     CK(cudaMemcpyAsync(m->d_bc_mask, bc_mask, sizeof(int) * n, cudaMemcpyHostToDevice, m->st));
     TRY(do_prepare(m, m->d_vals, m->d_res, m->d_dsol));
-    CK(cudaMemcpyAsync(vals, m->d_vals, sizeof(double) * m->nnz, cudaMemcpyDeviceToHost, m->st));
+    TRY(download(m, vals, m->d_vals, sizeof(double) * (size_t)m->nnz));
     CK(cudaMemcpyAsync(residual, m->d_res, sizeof(double) * n, cudaMemcpyDeviceToHost, m->st));
     CK(cudaMemcpyAsync(x, m->d_dsol, sizeof(double) * n, cudaMemcpyDeviceToHost, m->st));
     CK(cudaMemcpyAsync(bc_mask, m->d_bc_mask, sizeof(int) * n, cudaMemcpyDeviceToHost, m->st));
