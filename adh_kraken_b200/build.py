@@ -27,6 +27,7 @@ UNITS = [
     ("ilu_kernels.cu", []),
     ("amg_kernels.cu", []),
     ("gmres_kernels.cu", []),
+    ("small_kernels.cu", []),
     ("gnn_kernels.cu", []),
     ("sw2_capi.cu", []),
 ]

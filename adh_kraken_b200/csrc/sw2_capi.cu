@@ -44,6 +44,7 @@ extern "C" const char* sw2g_last_error(void) { return g_err.c_str(); }
 #define TRY(x) do { int r_ = (x); if (r_ != SW2G_OK) return r_; } while (0)
 
 static const int kChunk = 8;   // BiCGStab iterations per graph replay
+static const int kSmallChunk = 256;   // BiCGStab iterations per launch of the small meshes' solver
 static const double kPatchTileEdges = 7.0;   // tile side of the AMG chunk corrections, in mean edge lengths
 
 struct ProfRec { int cls; cudaEvent_t a, b; };
@@ -84,6 +85,9 @@ struct sw2g_model {
     double *d_sol = nullptr, *d_sol_old = nullptr, *d_sol_older = nullptr, *d_dirichlet = nullptr, *d_guess = nullptr;
     int *d_bc_mask = nullptr, *d_mask_save = nullptr;
     bool guess_set = false;
+    SmallPlan small;         // the small meshes' Krylov solver
+    std::vector<int> small_order;   // its order of the nodes
+    int small_m32 = 0;       // restart length of its last FP32 GMRES cycle
     bool can_undo = false;   // the levels were rotated by the last sw2g_step
     // work
     int *d_wd = nullptr, *d_node_tmp = nullptr;
@@ -297,6 +301,21 @@ static void build_csr(int V, int T, int S, const int* tri, const int* seg, std::
     }
 }
 
+// a level's rows in the small meshes' solver
+static int small_level(sw2g_model* m, int l, const std::vector<int>& bptr, const std::vector<int>& bcol, const std::vector<int>& order) {
+    const SmallHostLevel H = small_level_plan(bptr, bcol, order, m->small.ctas);
+    SmallLevelPlan& S = m->small.lev[l];
+    auto up = [&](const int** dst, const std::vector<int>& v) {
+        int* d = nullptr;
+        const int r = upload(m, &d, v.data(), v.size());
+        *dst = d;
+        return r;
+    };
+    TRY(up(&S.node, H.node)); TRY(up(&S.ptr, H.ptr)); TRY(up(&S.col, H.col)); TRY(up(&S.dptr, H.dptr)); TRY(up(&S.dst, H.dst));
+    S.slots = H.slots; S.halo = H.halo; S.push = H.push;
+    return SW2G_OK;
+}
+
 extern "C" void sw2g_default_opts(sw2g_newton_opts* o) {
     o->tol_nonlin = 1e-8; o->inc_nonlin = 1e-6; o->max_nonlin_it = 10; o->max_linesearch_cuts = 5;
     o->krylov_max_it = 4000; o->krylov_tol = 1e-11; o->krylov_precision = 64;
@@ -506,6 +525,16 @@ extern "C" int sw2g_create(const sw2g_mesh* mesh, void* cuda_stream, sw2g_model*
         cudaMallocHost((void**)&m->h_ks, sizeof(KrylovScalars)) != cudaSuccess ||
         cudaMallocHost((void**)&m->h_state, sizeof(int)) != cudaSuccess) {
         g_err = "cudaMallocHost failed"; return fail(SW2G_ERR_NOMEM);
+    }
+    if (V <= kClusterNodes) {
+        int limit = 0;
+        if (cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, m->device) != cudaSuccess) cudaGetLastError();
+        m->small = small_solver_plan(limit);
+        if (m->small.ctas > 0) {
+            m->small_order = small_order(m->h_bptr, m->h_bcol, V, m->small.ctas);
+            const int r = small_level(m, 0, m->h_bptr, m->h_bcol, m->small_order);
+            if (r != SW2G_OK) return fail(r);
+        }
     }
     if (sizeof(double) * (size_t)m->nnz >= kStageMin) {   // without the ring large downloads are plain copies
         if (cudaMallocHost((void**)&m->h_stage, kStageSlots * kStagePiece) != cudaSuccess) { cudaGetLastError(); m->h_stage = nullptr; }
@@ -812,6 +841,16 @@ static int build_amg(sw2g_model* m) {
         TRY(dalloc(m, &A.cl.op64, rows * rows)); TRY(dalloc(m, &A.cl.op32, rows * rows));
         while (A.cl.lo < A.nlev - 1 && A.lev[A.cl.lo].n > kClusterNodes) A.cl.lo++;
         A.cl.ctas = amg_cluster_ctas();
+        std::vector<int> order = m->small_order;
+        for (int l = 0; l < A.nlev - 1 && m->small.ctas > 0; l++) {
+            const std::vector<int> coarse = small_coarse_order(order, K[l].agg, L[l + 1].n);
+            const SmallHostLink H = small_link_plan(K[l].agg, K[l].mptr, K[l].mem, order, coarse, l + 2 == A.nlev, m->small.ctas);
+            SmallLevelPlan& S = m->small.lev[l];
+            TRY(up(&S.agg, H.agg)); TRY(up(&S.mptr, H.mptr)); TRY(up(&S.mem, H.mem));
+            S.members = H.members;
+            order = coarse;
+            TRY(small_level(m, l + 1, L[l + 1].bptr, L[l + 1].bcol, order));
+        }
     }
     m->amg_ready = true;
     static const bool trace = getenv("SW2G_TRACE_KRYLOV") != nullptr;
@@ -965,14 +1004,16 @@ static int run_bicg(sw2g_model* m, KrylovVecs<VT> V, int precond, cudaGraphExec_
     op.kind = precond; op.ilu = &m->ilu; op.lu = V.vals_pc; op.dinv = V.inv; op.amg = &m->amg; op.vals = V.vals;
     op.right = precond == SW2G_PC_AMG;
     const int per_apply = precond == SW2G_PC_BILU0 ? 2 * m->ilu.ncolors : precond_launches(m, precond);
+    const bool small = pc && small_solver_takes<VT>(m->B, op, m->small, 0);
     {
-        ProfScope ps(m, 4, pc ? 3 + 2 * per_apply : 2);
+        ProfScope ps(m, 4, small ? 1 : pc ? 3 + 2 * per_apply : 2);
         CK(cudaMemcpyAsync(m->d_ks, &init, sizeof(KrylovScalars), cudaMemcpyHostToDevice, m->st));
-        if (pc) launch_bicg_init_pc<VT>(m->B, op, V, m->d_ks, R, m->st);
+        if (small) small_bicg<VT>(m->B, op, V, m->d_ks, true, kSmallChunk, m->small, m->st);
+        else if (pc) launch_bicg_init_pc<VT>(m->B, op, V, m->d_ks, R, m->st);
         else launch_bicg_init<VT>(m->B, V, m->d_ks, R, m->st);
         CKL();
     }
-    if (!*graph) {
+    if (!small && !*graph) {
         cudaGraph_t g;
         CK(cudaStreamBeginCapture(m->st, cudaStreamCaptureModeThreadLocal));
         for (int c = 0; c < kChunk; c++) {
@@ -997,8 +1038,13 @@ static int run_bicg(sw2g_model* m, KrylovVecs<VT> V, int precond, cudaGraphExec_
             fprintf(stderr, "krylov it %d rnorm %.3e bnorm %.3e rel %.3e\n", m->h_ks->it, m->h_ks->rnorm, m->h_ks->bnorm,
                     m->h_ks->rnorm / (m->h_ks->bnorm > 0 ? m->h_ks->bnorm : 1.0));
         if (m->h_ks->done) break;
-        ProfScope ps(m, 4, per_it * kChunk);
-        CK(cudaGraphLaunch(*graph, m->st));
+        ProfScope ps(m, 4, small ? 1 : per_it * kChunk);
+        if (small) {
+            small_bicg<VT>(m->B, op, V, m->d_ks, false, kSmallChunk, m->small, m->st);
+            CKL();
+        } else {
+            CK(cudaGraphLaunch(*graph, m->st));
+        }
     }
     if (op.right) {   // x holds y of A M^-1 y = b: x = M^-1 y
         ProfScope ps(m, 4, per_apply);
@@ -1167,18 +1213,18 @@ static int run_cycle(sw2g_model* m, const CycleGraph& C, int per_step, bool whol
 }
 // FP32 cycle: FP32 basis, FP32 matrix and FP32 preconditioner on the FP32 right-hand side f_b; the
 // correction lands in f_x (the FP64 residual and the update stay with the caller)
-static int gmres_graph32(sw2g_model* m, int precond, int mres) {
+static PrecondOp<float> gmres_precond32(sw2g_model* m, int precond) {
     PrecondOp<float> op;
     op.kind = precond; op.right = true; op.ilu = &m->ilu; op.lu = m->f_lu; op.dinv = m->f_inv; op.amg = &m->amg;
     op.vals = m->f_vals;
-    return build_cycle<float>(m, &m->gm_cycle_b32, op, m->f_vals, m->gm_V32, m->f_z, m->f_b, m->f_x, mres);
+    return op;
 }
-static int gmres_graph(sw2g_model* m, bool mixed, int precond, int mres) {
+static PrecondOp<double> gmres_precond(sw2g_model* m, bool mixed, int precond) {
     PrecondOp<double> op;
     op.kind = precond; op.right = true; op.ilu = &m->ilu; op.lu = m->d_lu; op.dinv = m->d_inv; op.amg = &m->amg;
     op.vals = m->d_vals;
     if (mixed) { op.mixed = true; op.vals32 = m->f_vals; op.lu32 = m->f_lu; op.dinv32 = m->f_inv; op.tmp32 = m->f_z; }
-    return build_cycle<double>(m, mixed ? &m->gm_cycle32 : &m->gm_cycle64, op, m->d_vals, m->gm_V64, m->k_z, m->d_t64, m->k_xi, mres);
+    return op;
 }
 
 // Restarted GMRES(kGmM) on the prepared (scaled) system, FP64 Krylov basis.  Each
@@ -1217,18 +1263,25 @@ static int solve_gmres(sw2g_model* m, double* x, double* b, const sw2g_newton_op
         CKL();
     }
     const bool basis32 = mixed && o.krylov_basis_precision == 32;
+    bool small = false;   // a cycle is one kernel (small_kernels.cu)
     if (basis32) {
         if (!m->gm_V32 || m->gm_cap32 < mres) {
             TRY(gmres_basis(m, &m->gm_V32, &m->gm_cap32, mres));
             m->gm_cycle_b32.clear();   // the cycle's graphs hold the old basis address
         }
-        TRY(gmres_graph32(m, o.precond, mres));
+        small = small_solver_takes<float>(m->B, gmres_precond32(m, o.precond), m->small, mres) && !gm_reorth();
+        if (small) m->small_m32 = mres;
+        else
+            TRY(build_cycle<float>(m, &m->gm_cycle_b32, gmres_precond32(m, o.precond), m->f_vals, m->gm_V32, m->f_z, m->f_b, m->f_x, mres));
     } else {
         if (!m->gm_V64 || m->gm_cap64 < mres) {
             TRY(gmres_basis(m, &m->gm_V64, &m->gm_cap64, mres));
             m->gm_cycle32.clear(); m->gm_cycle64.clear();
         }
-        TRY(gmres_graph(m, mixed, o.precond, mres));
+        small = small_solver_takes<double>(m->B, gmres_precond(m, mixed, o.precond), m->small, mres) && !gm_reorth();
+        if (!small)
+            TRY(build_cycle<double>(m, mixed ? &m->gm_cycle32 : &m->gm_cycle64, gmres_precond(m, mixed, o.precond), m->d_vals,
+                                    m->gm_V64, m->k_z, m->d_t64, m->k_xi, mres));
     }
     const int pl = precond_launches(m, o.precond) + (mixed ? 2 : 0);
     const int per_step = 4 + pl;
@@ -1290,13 +1343,17 @@ static int solve_gmres(sw2g_model* m, double* x, double* b, const sw2g_newton_op
         if (rtol < (basis32 ? 1e-5 : 1e-12)) rtol = basis32 ? 1e-5 : 1e-12;   // FP32 resolves no more per cycle
         CK(cudaMemcpyAsync(m->gm.scal + 3, &rtol, sizeof(double), cudaMemcpyHostToDevice, m->st));
         {
-            ProfScope ps(m, 4, 5 + pl + (basis32 ? 2 : 0));   // besides the steps
+            ProfScope ps(m, 4, (small ? 2 : 5 + pl) + (basis32 ? 2 : 0));   // besides the steps
             if (basis32) {   // FP32 Krylov cycle inside the FP64 refinement
                 launch_to_float(n, m->d_t64, m->f_b, m->st);
-                TRY(run_cycle(m, m->gm_cycle_b32, per_step, false));
+                if (small) small_gmres_cycle<float>(m->B, gmres_precond32(m, o.precond), m->f_vals, m->gm_V32, gm_ld(n), m->f_b,
+                                                    m->f_x, m->gm_rw, m->gm, mres, m->small, m->st);
+                else TRY(run_cycle(m, m->gm_cycle_b32, per_step, false));
                 launch_to_double(n, m->f_x, m->k_xi, m->st);
             } else {
-                TRY(run_cycle(m, mixed ? m->gm_cycle32 : m->gm_cycle64, per_step, false));
+                if (small) small_gmres_cycle<double>(m->B, gmres_precond(m, mixed, o.precond), m->d_vals, m->gm_V64, gm_ld(n),
+                                                     m->d_t64, m->k_xi, m->gm_rw, m->gm, mres, m->small, m->st);
+                else TRY(run_cycle(m, mixed ? m->gm_cycle32 : m->gm_cycle64, per_step, false));
             }
             launch_axpy(n, 1.0, m->k_xi, x, m->st);
             CKL();
@@ -1864,7 +1921,7 @@ extern "C" int sw2g_reset_profile(sw2g_model* m) {
 
 extern "C" int sw2g_time_kernel(sw2g_model* m, int which, int reps, double* avg_ms, double* bytes) {
     NEED(m && avg_ms && bytes && reps > 0 && which >= 0 && which <= 9, "sw2g_time_kernel: bad argument");
-    NEED(which != 8 || m->gm_cycle_b32.m > 0, "sw2g_time_kernel: no FP32 GMRES cycle has run yet");
+    NEED(which != 8 || m->gm_cycle_b32.m > 0 || m->small_m32 > 0, "sw2g_time_kernel: no FP32 GMRES cycle has run yet");
     const double nnz = m->nnz, n = m->n, T = m->T, S = m->S;
     if (which >= 4) {   // the AMG sweeps
         if (!m->amg_ready) TRY(build_amg(m));
@@ -1887,7 +1944,10 @@ extern "C" int sw2g_time_kernel(sw2g_model* m, int which, int reps, double* avg_
             case 7: spmv_skip<float>(m->B, m->f_vals, m->f_p, m->f_Ap, nullptr, nullptr, m->st); break;
             case 8:   // a whole FP32 GMRES cycle with its stopping test off: every iteration runs
                 cudaMemcpyAsync(m->gm.scal + 3, &zero, sizeof(double), cudaMemcpyHostToDevice, m->st);
-                run_cycle(m, m->gm_cycle_b32, 0, true);
+                if (m->small_m32 > 0)
+                    small_gmres_cycle<float>(m->B, gmres_precond32(m, SW2G_PC_AMG), m->f_vals, m->gm_V32, gm_ld(m->n), m->f_b,
+                                             m->f_x, m->gm_rw, m->gm, m->small_m32, m->small, m->st);
+                else run_cycle(m, m->gm_cycle_b32, 0, true);
                 break;
             case 9: amg_patch_correct<float>(m->B, m->amg, m->f_vals, m->f_p, m->f_Ap, nullptr, m->st); break;
 
@@ -1914,7 +1974,7 @@ extern "C" int sw2g_time_kernel(sw2g_model* m, int which, int reps, double* avg_
         case 6: *bytes = 4.0 * (8.0 * nnz + 32.0 * n); break;   // ~4 level-0 matrix passes (coarse levels extra)
         case 5: *bytes = 8.0 * nnz + 12.0 * n + 12.0 * n + 8.0 * n; break;   // FP32 SpMV + FP32 block apply
         case 7: *bytes = 8.0 * nnz + 12.0 * n; break;                        // FP32 values + cols, x and y
-        case 8: *bytes = (double)m->gm_cycle_b32.m; break;                          // iterations of the cycle (not bytes)
+        case 8: *bytes = (double)(m->small_m32 > 0 ? m->small_m32 : m->gm_cycle_b32.m); break;                          // iterations of the cycle (not bytes)
         case 9: *bytes = 4.0 * (double)m->p_rtot + 12.0 * m->p_nentries; break;   // FP32 inverse rows + residuals
     }
     return SW2G_OK;

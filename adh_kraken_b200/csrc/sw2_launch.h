@@ -1,5 +1,6 @@
 // Host-side launchers of the SW2 and linear-algebra kernels.
 #pragma once
+#include <vector>
 #include <cuda_runtime.h>
 #include "sw2_device.h"
 
@@ -257,6 +258,35 @@ void gmres_steps(const BlockCSR& A, const PrecondOp<VT>& P, const VT* vals, VT* 
                  const GmresDev& G, cudaStream_t st, int first, int last, bool reorth);
 template <class VT>
 void gmres_end(const BlockCSR& A, const PrecondOp<VT>& P, VT* Vb, size_t ld, VT* z, VT* out, const GmresDev& G, cudaStream_t st);
+// ---- Krylov solves of small meshes in one thread-block cluster (small_kernels.cu)
+struct SmallHostLevel { std::vector<int> node, ptr, col, dptr, dst; int slots = 0, halo = 0, push = 0; };
+struct SmallHostLink { std::vector<int> agg, mptr, mem; int members = 0; };
+std::vector<int> small_order(const std::vector<int>& bptr, const std::vector<int>& bcol, int n, int ctas);
+std::vector<int> small_coarse_order(const std::vector<int>& fine, const std::vector<int>& agg, int nc);
+SmallHostLevel small_level_plan(const std::vector<int>& bptr, const std::vector<int>& bcol, const std::vector<int>& order, int ctas);
+SmallHostLink small_link_plan(const std::vector<int>& agg, const std::vector<int>& mptr, const std::vector<int>& mem,
+                              const std::vector<int>& order, const std::vector<int>& coarse, bool coarsest, int ctas);
+struct SmallLevelPlan {                 // nodes in the cluster's order, rows, and of the nodes of one CTA:
+    const int *node, *ptr;
+    const int *col, *dptr, *dst;        // neighbour slots' indices in its vectors (own entries, then its copies of others);
+                                        // the copies of each node, CTA << 16 | index
+    const int *agg, *mptr, *mem;        // aggregates and their members, CTA << 16 | index
+    int slots, halo, push, members;     // the most slots, copies held, copies to write and members of a CTA
+};
+struct SmallPlan {
+    int ctas = 0;                       // CTAs of the cluster, 0: not for this mesh or device
+    int smem = 0;                       // dynamic shared memory a CTA may use
+    SmallLevelPlan lev[kAmgMaxLevels] = {};
+};
+SmallPlan small_solver_plan(int smem_limit);
+template <class VT>   // restart: of GMRES, 0 for BiCGStab
+bool small_solver_takes(const BlockCSR& A, const PrecondOp<VT>& op, const SmallPlan& S, int restart);
+template <class VT>   // a whole GMRES cycle, the same buffers and results as gmres_begin .. gmres_end
+void small_gmres_cycle(const BlockCSR& A, const PrecondOp<VT>& op, const VT* vals, VT* Vb, size_t ld, const VT* rhs, VT* out,
+                       const double* rw, const GmresDev& G, int m, const SmallPlan& plan, cudaStream_t st);
+template <class VT>   // the start of a preconditioned BiCGStab solve (first) and up to `iterations` iterations
+void small_bicg(const BlockCSR& A, const PrecondOp<VT>& op, const KrylovVecs<VT>& V, KrylovScalars* S, bool first, int iterations,
+                const SmallPlan& plan, cudaStream_t st);
 // rw_i = 1 / s_i (weights that make a scaled system's residual the unscaled one)
 void launch_inv_scale(int n, const double* scale, double* rw, cudaStream_t st);
 template <class VT>
