@@ -43,9 +43,8 @@ __device__ __forceinline__ bool gm_last_block(const GmresDev& G) {
     __threadfence();   // every thread's partial writes are visible device-wide before the count
     __syncthreads();
     if (threadIdx.x == 0) {
-        const unsigned int total = gridDim.x * gridDim.y;
-        unsigned int t = atomicInc(G.counter, total - 1);
-        is_last = (t == total - 1);
+        unsigned int t = atomicInc(G.counter, gridDim.x - 1);
+        is_last = (t == gridDim.x - 1);
     }
     __syncthreads();
     return is_last;
@@ -83,7 +82,7 @@ __device__ __forceinline__ void st16(double* p, const double (&o)[2]) {
 __device__ __forceinline__ double gm_sum_partials(const GmresDev& G, int col) {
     __shared__ double red[8];
     double t = 0;
-    for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) t += __ldcg(G.partial + b * (kGmM + 1) + col);
+    for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) t += __ldcg(G.partial + col * kMaxBlocks + b);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = t;
@@ -111,7 +110,7 @@ __global__ void __launch_bounds__(256) k_gm_start(int n, const VT* __restrict__ 
     if (threadIdx.x == 0) {
         double t = 0;
         for (int k = 0; k < 8; k++) t += sh[k];
-        G.partial[blockIdx.x * (kGmM + 1)] = t;
+        G.partial[blockIdx.x] = t;
     }
     if (!gm_last_block(G)) return;
     const double tsum = gm_sum_partials(G, 0);
@@ -137,65 +136,89 @@ __global__ void k_gm_v0(int n, const VT* __restrict__ r, const double* __restric
 }
 
 // h_k = v_k . w for k < nv (w = v_nv before orthogonalisation), into column j of H.
-// blockIdx.y picks a group of kDotGroup basis vectors: each thread keeps kDotGroup
-// accumulators (about 40 registers instead of one per basis vector), so 6 blocks fit on
-// an SM and every load of the group is issued at once.  A thread's elements and the
-// reduction tree do not depend on the group, so every h_k is the same sum as with all
-// accumulators in one thread.  w is read once per group.
+// A block takes kDotGroup basis vectors at a time: their 16-byte loads are issued together, and each thread keeps an accumulator
+// for each.  A thread's elements and the reduction tree do not depend on the group, so every h_k is the same sum as with all
+// accumulators in one thread; w comes from L2 for every group but the first.
+// On a small mesh a block has one load per thread and vector, and what bounded it was its own end (a tree of 40 shuffles, a
+// fence, a count) as one block per group, with the sum over the blocks left to one of all blocks, from partials a column's width
+// apart: 19.6 us at 188k FP64 entries and 58 us at 1.5M FP32 ones (means over cycles of 30 and 50 steps), now 11.5
+// and 44 us.  The eight trees share their shuffles: at each level a lane keeps half of the columns and hands the others to its
+// partner, and each column's tree stays the same.
+// Four blocks on an SM hold the whole grid (592 blocks) at once: with the three that its registers allowed freely the FP32
+// case took 51 us.
 constexpr int kDotGroup = 8;
+constexpr int kDotLoads = 10;   // partials a lane loads at once: half of a full grid's 592 / 32
+template <int O, int K>
+__device__ __forceinline__ void dot_level(double* acc) {   // K columns -> K / 2, the upper ones where lane & O
+    const bool up = threadIdx.x & O;
+#pragma unroll
+    for (int k = 0; k < K / 2; k++) {
+        const double keep = up ? acc[k + K / 2] : acc[k], give = up ? acc[k] : acc[k + K / 2];
+        acc[k] = keep + __shfl_xor_sync(0xffffffffu, give, O);
+    }
+}
 template <class VT>
-__global__ void __launch_bounds__(256) k_gm_dots(int n, int nv, const VT* __restrict__ Vb, size_t ld, double* dst,
+__global__ void __launch_bounds__(256, 4) k_gm_dots(int n, int nv, const VT* __restrict__ Vb, size_t ld, double* dst,
                                                  GmresDev G) {
     if (G.state[0]) return;
-    __shared__ double sh[8][kDotGroup];
-    const int k0 = blockIdx.y * kDotGroup;
+    __shared__ double sh[2][8][kDotGroup];
     const VT* w = Vb + (size_t)nv * ld;
-    double acc[kDotGroup];
-#pragma unroll
-    for (int k = 0; k < kDotGroup; k++) acc[k] = 0.0;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     constexpr int NQ = Quad<VT>::N;
     const int nq = n / NQ;
-    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < nq; q += gridDim.x * blockDim.x) {
-        const size_t i = (size_t)q * NQ;
-        VT wq[NQ];
-        ld16_rw(w + i, wq);
-        VT x[kDotGroup][NQ];
+    for (int k0 = 0, turn = 0; k0 < nv; k0 += kDotGroup, turn ^= 1) {
+        double acc[kDotGroup];
 #pragma unroll
-        for (int k = 0; k < kDotGroup; k++)
-            if (k0 + k < nv) ld16(Vb + (size_t)(k0 + k) * ld + i, x[k]);
+        for (int k = 0; k < kDotGroup; k++) acc[k] = 0.0;
+        for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < nq; q += gridDim.x * blockDim.x) {
+            const size_t i = (size_t)q * NQ;
+            VT wq[NQ];
+            ld16_rw(w + i, wq);
+            VT x[kDotGroup][NQ];
 #pragma unroll
-        for (int k = 0; k < kDotGroup; k++)
-            if (k0 + k < nv) {
+            for (int k = 0; k < kDotGroup; k++)
+                if (k0 + k < nv) ld16(Vb + (size_t)(k0 + k) * ld + i, x[k]);
 #pragma unroll
-                for (int c = 0; c < NQ; c++) acc[k] += (double)x[k][c] * (double)wq[c];
-            }
-    }
-    for (int i = nq * NQ + blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const double wi = w[i];
+            for (int k = 0; k < kDotGroup; k++)
+                if (k0 + k < nv) {
 #pragma unroll
-        for (int k = 0; k < kDotGroup; k++)
-            if (k0 + k < nv) acc[k] += (double)Vb[(size_t)(k0 + k) * ld + i] * wi;
-    }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+                    for (int c = 0; c < NQ; c++) acc[k] += (double)x[k][c] * (double)wq[c];
+                }
+        }
+        for (int i = nq * NQ + blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+            const double wi = w[i];
 #pragma unroll
-    for (int k = 0; k < kDotGroup; k++) {
-        if (k0 + k < nv) {
-            double v = acc[k];
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            if (lane == 0) sh[warp][k] = v;
+            for (int k = 0; k < kDotGroup; k++)
+                if (k0 + k < nv) acc[k] += (double)Vb[(size_t)(k0 + k) * ld + i] * wi;
+        }
+        dot_level<16, 8>(acc);
+        dot_level<8, 4>(acc);
+        dot_level<4, 2>(acc);
+        double v = acc[0];                          // column lane >> 2, bit by bit
+        v += __shfl_xor_sync(0xffffffffu, v, 2);
+        v += __shfl_xor_sync(0xffffffffu, v, 1);
+        if ((lane & 3) == 0) sh[turn][warp][lane >> 2] = v;
+        __syncthreads();
+        if (threadIdx.x < kDotGroup && k0 + (int)threadIdx.x < nv) {
+            double t = 0;
+            for (int w8 = 0; w8 < 8; w8++) t += sh[turn][w8][threadIdx.x];
+            G.partial[(k0 + threadIdx.x) * kMaxBlocks + blockIdx.x] = t;
         }
     }
-    __syncthreads();
-    if (threadIdx.x < kDotGroup && k0 + (int)threadIdx.x < nv) {
-        double t = 0;
-        for (int w8 = 0; w8 < 8; w8++) t += sh[w8][threadIdx.x];
-        G.partial[blockIdx.x * (kGmM + 1) + k0 + threadIdx.x] = t;
-    }
     if (gm_last_block(G)) {   // warp w sums columns w, w + 8, ...; its lanes stride over the blocks
-        for (int c = warp; c < nv; c += (int)(blockDim.x >> 5)) {
+        for (int c = warp; c < nv; c += 8) {
             double t = 0;
-            for (int b = lane; b < (int)gridDim.x; b += 32) t += __ldcg(G.partial + b * (kGmM + 1) + c);
+            for (int b0 = lane; b0 < (int)gridDim.x; b0 += 32 * kDotLoads) {
+                double p[kDotLoads];
+#pragma unroll
+                for (int u = 0; u < kDotLoads; u++) {
+                    const int b = b0 + 32 * u;
+                    p[u] = b < (int)gridDim.x ? __ldcg(G.partial + c * kMaxBlocks + b) : 0.0;
+                }
+#pragma unroll
+                for (int u = 0; u < kDotLoads; u++)
+                    if (b0 + 32 * u < (int)gridDim.x) t += p[u];
+            }
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
             if (lane == 0) dst[c] = t;
@@ -288,7 +311,7 @@ __global__ void __launch_bounds__(256) k_gm_orth(int n, int j, VT* __restrict__ 
     if (threadIdx.x == 0) {
         double t = 0;
         for (int k = 0; k < 8; k++) t += sh[k];
-        G.partial[blockIdx.x * (kGmM + 1)] = t;
+        G.partial[blockIdx.x] = t;
     }
     if (!gm_last_block(G)) return;
     // the column and the earlier rotations in shared memory: one thread applies them in turn, and each step from
@@ -410,11 +433,10 @@ void gmres_steps(const BlockCSR& A, const PrecondOp<VT>& P, const VT* vals, VT* 
     for (int j = first; j < last; j++) {
         precond_apply<VT>(A, P, Vb + (size_t)j * ld, z, done, st);
         spmv_skip<VT>(A, vals, z, Vb + (size_t)(j + 1) * ld, rw, done, st);
-        const dim3 dg(g, (j + 1 + kDotGroup - 1) / kDotGroup);
-        k_gm_dots<VT><<<dg, 256, 0, st>>>(n, j + 1, Vb, ld, G.H + (size_t)j * (kGmM + 1), G);
+        k_gm_dots<VT><<<g, 256, 0, st>>>(n, j + 1, Vb, ld, G.H + (size_t)j * (kGmM + 1), G);
         if (reorth) {
             k_gm_sub<VT><<<g, 256, 0, st>>>(n, j, Vb, ld, G);
-            k_gm_dots<VT><<<dg, 256, 0, st>>>(n, j + 1, Vb, ld, G.H2, G);
+            k_gm_dots<VT><<<g, 256, 0, st>>>(n, j + 1, Vb, ld, G.H2, G);
             k_gm_orth<VT, true><<<g, 256, 0, st>>>(n, j, Vb, ld, G);
         } else {
             k_gm_orth<VT, false><<<g, 256, 0, st>>>(n, j, Vb, ld, G);

@@ -244,7 +244,7 @@ struct GmresDev {                       // device buffers of one cycle
     double* cs = nullptr; double* sn = nullptr;   // [kGmM] Givens rotations
     double* g = nullptr;                // [kGmM+1] rotated right-hand side
     double* y = nullptr;                // [kGmM] least-squares solution
-    double* partial = nullptr;          // [kMaxBlocks*(kGmM+1)] block partials
+    double* partial = nullptr;          // [kGmM+1][kMaxBlocks] block partials
     unsigned int* counter = nullptr;    // last-block counter (wraps to 0)
     int* state = nullptr;               // [0] done, [1] columns built, [2] status (0 ok, 1 breakdown, 2 non-finite)
     double* scal = nullptr;             // [0] beta, [1] target, [2] residual estimate, [3] rtol (host-set), [4] h_{j+1,j}
