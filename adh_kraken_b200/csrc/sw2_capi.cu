@@ -985,10 +985,10 @@ static int build_patches(sw2g_model* m, const double* vals) {
 // kernel launches of one preconditioner application (profiling counts)
 static int precond_launches(const sw2g_model* m, int precond) {
     if (precond == SW2G_PC_BILU0) return 2 * m->ilu.ncolors;
-    if (precond == SW2G_PC_AMG) {   // per level: 2 kAmgNu sweeps, residual, restriction, prolongation
+    if (precond == SW2G_PC_AMG) {   // per level: 2 kAmgNu sweeps, residual, restriction (with the next level's first sweep), prolongation
         const AmgHost& H = m->amg;
         const int lo = H.cl.ctas == 0 ? H.nlev - 1 : (H.cl.lo == 0 && H.patch.mode == 2) ? 1 : H.cl.lo;
-        return lo * (2 * kAmgNu + 3) + 1 + 2 * H.patch.mode;
+        return lo * (2 * kAmgNu + 3) - std::max(0, lo - 1) + 1 + 2 * H.patch.mode;
     }
     return 1;
 }
