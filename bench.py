@@ -480,7 +480,7 @@ def run_ours(args, world, rank, local, dist):
         "fast_detail": sf,
         "gpu_launches": int(np.sum(prof_n)),
         "clocks": clocks,
-        "roofline": {"kernel": "k_amg_l0<float,1,2> (AMG level-0 smoothing sweep, FP32)", "bound": "hbm",
+        "roofline": {"kernel": "k_tile_rows<1> (AMG level-0 smoothing sweep, FP32)", "bound": "hbm",
                      "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
                      "peak_source": peak_src, "traffic": traffic, "algorithmic_bytes": rf_bytes,
                      "avg_launch_ms": rf_ms,
