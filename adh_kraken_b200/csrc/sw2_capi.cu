@@ -87,7 +87,7 @@ struct sw2g_model {
     bool guess_set = false;
     SmallPlan small;         // the small meshes' Krylov solver
     std::vector<int> small_order;   // its order of the nodes
-    int small_m32 = 0;       // restart length of its last FP32 GMRES cycle
+    int small_m32 = 0, small_pc32 = 0;   // restart length and preconditioner of its last FP32 GMRES cycle
     bool can_undo = false;   // the levels were rotated by the last sw2g_step
     // work
     int *d_wd = nullptr, *d_node_tmp = nullptr;
@@ -1270,8 +1270,9 @@ static int solve_gmres(sw2g_model* m, double* x, double* b, const sw2g_newton_op
             m->gm_cycle_b32.clear();   // the cycle's graphs hold the old basis address
         }
         small = small_solver_takes<float>(m->B, gmres_precond32(m, o.precond), m->small, mres) && !gm_reorth();
-        if (small) m->small_m32 = mres;
-        else
+        m->small_m32 = small ? mres : 0;
+        m->small_pc32 = o.precond;
+        if (!small)
             TRY(build_cycle<float>(m, &m->gm_cycle_b32, gmres_precond32(m, o.precond), m->f_vals, m->gm_V32, m->f_z, m->f_b, m->f_x, mres));
     } else {
         if (!m->gm_V64 || m->gm_cap64 < mres) {
@@ -1945,7 +1946,7 @@ extern "C" int sw2g_time_kernel(sw2g_model* m, int which, int reps, double* avg_
             case 8:   // a whole FP32 GMRES cycle with its stopping test off: every iteration runs
                 cudaMemcpyAsync(m->gm.scal + 3, &zero, sizeof(double), cudaMemcpyHostToDevice, m->st);
                 if (m->small_m32 > 0)
-                    small_gmres_cycle<float>(m->B, gmres_precond32(m, SW2G_PC_AMG), m->f_vals, m->gm_V32, gm_ld(m->n), m->f_b,
+                    small_gmres_cycle<float>(m->B, gmres_precond32(m, m->small_pc32), m->f_vals, m->gm_V32, gm_ld(m->n), m->f_b,
                                              m->f_x, m->gm_rw, m->gm, m->small_m32, m->small, m->st);
                 else run_cycle(m, m->gm_cycle_b32, 0, true);
                 break;
@@ -1974,7 +1975,7 @@ extern "C" int sw2g_time_kernel(sw2g_model* m, int which, int reps, double* avg_
         case 6: *bytes = 4.0 * (8.0 * nnz + 32.0 * n); break;   // ~4 level-0 matrix passes (coarse levels extra)
         case 5: *bytes = 8.0 * nnz + 12.0 * n + 12.0 * n + 8.0 * n; break;   // FP32 SpMV + FP32 block apply
         case 7: *bytes = 8.0 * nnz + 12.0 * n; break;                        // FP32 values + cols, x and y
-        case 8: *bytes = (double)(m->small_m32 > 0 ? m->small_m32 : m->gm_cycle_b32.m); break;                          // iterations of the cycle (not bytes)
+        case 8: *bytes = (double)(m->small_m32 > 0 ? m->small_m32 : m->gm_cycle_b32.m); break;   // iterations of the cycle (not bytes)
         case 9: *bytes = 4.0 * (double)m->p_rtot + 12.0 * m->p_nentries; break;   // FP32 inverse rows + residuals
     }
     return SW2G_OK;
