@@ -580,9 +580,14 @@ static int num_sms() {
 }
 static bool dense_sizes(int in, int out) { return in > 0 && in <= MAXIN && out > 0 && out <= H && in % 4 == 0; }
 extern "C++" {
-template <class K> static bool dense_attr(K kernel, size_t smem) {
-    return smem <= 48 * 1024 || cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess;
+// Allows a launch of `smem` bytes.  What is set is always `most`, the kernel's need at the widest layer: the attribute is the
+// kernel's, not the launch's, and a thread that set its own smaller need would have another's launch refused.
+template <class K> static bool dense_attr(K kernel, size_t smem, size_t most) {
+    return smem <= 48 * 1024 || cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) == cudaSuccess;
 }
+static constexpr size_t fwd_smem(int in, int npt) { return sizeof(float) * ((size_t)in * H + 2 * 16 * (size_t)npt * LDA); }
+static constexpr size_t bwd_smem(int in, int out, int npt) { return sizeof(float) * ((size_t)((out + 3) & ~3) * in + (size_t)16 * npt * (H + 4)); }
+static constexpr size_t narrow_smem(int in) { return sizeof(float) * ((size_t)in * NARROW + (size_t)NARROW_NODES * (in + 1)); }
 }
 // Tiles of 128 nodes from one per SM on; below that tiles of 16 nodes, which spread a small graph over more SMs
 // (1600 nodes, forward of all layers: 242 us with 64-node tiles, 47 us with 16).
@@ -592,9 +597,9 @@ extern "C++" {
 template <int NPT>
 static int run_dense_fwd(int n, int in, int out, const __nv_bfloat16* W, const float* b, const float* X, const float* R, int act,
                          float* Z, float* Y, int vec, int sms, cudaStream_t st) {
-    const size_t smem = sizeof(float) * ((size_t)in * H + 2 * 16 * NPT * LDA);
+    const size_t smem = fwd_smem(in, NPT);
     const int tiles = nb(n, 16 * NPT), grid = tiles < 2 * sms ? tiles : 2 * sms;
-    if (!dense_attr(k_dense_fwd<NPT>, smem)) return -2;
+    if (!dense_attr(k_dense_fwd<NPT>, smem, fwd_smem(MAXIN, NPT))) return -2;
     k_dense_fwd<NPT><<<grid, DENSE_THREADS, smem, st>>>(n, in, out, W, b, X, R, act, Z, Y, vec);
     return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
@@ -605,8 +610,8 @@ int sw2n_dense_fwd(int n, int in, int out, const void* W_bf16, const float* b, c
     const __nv_bfloat16* W = (const __nv_bfloat16*)W_bf16;
     cudaStream_t st = (cudaStream_t)stream;
     if (out <= NARROW) {
-        const size_t smem = sizeof(float) * ((size_t)in * NARROW + (size_t)NARROW_NODES * (in + 1));
-        if (!dense_attr(k_dense_narrow, smem)) return -2;
+        const size_t smem = narrow_smem(in);
+        if (!dense_attr(k_dense_narrow, smem, narrow_smem(MAXIN))) return -2;
         k_dense_narrow<<<nb(n, NARROW_NODES), NARROW_NODES, smem, st>>>(n, in, out, W, b, X, R, act, Z, Y);
         return cudaGetLastError() == cudaSuccess ? 0 : -2;
     }
@@ -621,9 +626,9 @@ extern "C++" {
 template <int NPT>
 static bool run_dense_bwd_x(int n, int in, int out, const __nv_bfloat16* W, const float* Z, const float* dY, int act, float* dZ,
                             float* dX, int vec, int sms, cudaStream_t st) {
-    const size_t smem = sizeof(float) * ((size_t)((out + 3) & ~3) * in + (size_t)16 * NPT * (H + 4));
+    const size_t smem = bwd_smem(in, out, NPT);
     const int tiles = nb(n, 16 * NPT), grid = tiles < 2 * sms ? tiles : 2 * sms;
-    if (!dense_attr(k_dense_bwd_x<NPT>, smem)) return false;
+    if (!dense_attr(k_dense_bwd_x<NPT>, smem, bwd_smem(MAXIN, H, NPT))) return false;
     k_dense_bwd_x<NPT><<<grid, DENSE_THREADS, smem, st>>>(n, in, out, W, Z, dY, act, dZ, dX, vec);
     return true;
 }
