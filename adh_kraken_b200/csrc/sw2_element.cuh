@@ -154,11 +154,13 @@ __device__ __forceinline__ void cut_redistribute(const Cut& c, const V2 x[3], do
 // Apply the wrapper's rule around an integrand `f(rhs, x, h, ...)`.  `sub(nr)` must
 // evaluate the integrand on the sub-triangle described by the Cut.  Returns the
 // wrapper's wet fraction.
-// WET: all three depths are known to be positive.
-template <bool WET, class Full, class Sub>
+// STATE: what is known of the three depths.
+enum { ANY = 0, ALL_WET = 1, ALL_DRY = 2 };   // nothing; all positive; none positive
+template <int STATE, class Full, class Sub>
 __device__ __forceinline__ double wd_wrap(double r[9], const V2 x[3], const double h[3], double djac, bool redist,
                                           Full full, Sub sub) {
-    if (WET) { full(r); return 1.0; }
+    if (STATE == ALL_WET) { full(r); return 1.0; }
+    if (STATE == ALL_DRY) return 0.0;
     int only;
     int total = classify(h, &only);
     if (total == 3) return 0.0;
@@ -178,9 +180,10 @@ __device__ __forceinline__ double wd_wrap(double r[9], const V2 x[3], const doub
 }
 
 // fe_sw2_wet_dry_factor, fe_wet_dry_wrapper.c:29
-template <bool WET>
+template <int STATE>
 __device__ __forceinline__ double wd_factor(const V2 x[3], const double h[3], double djac) {
-    if (WET) return 1.0;
+    if (STATE == ALL_WET) return 1.0;
+    if (STATE == ALL_DRY) return 0.0;
     int only;
     int total = classify(h, &only);
     if (total == 3) return 0.0;
@@ -314,11 +317,11 @@ __device__ __forceinline__ void ig_gls_convection(double r[9], const V2 g[3], do
 
 // ----------------------------------------------------------------------------
 // wrapped terms
-template <bool WET>
+template <int STATE>
 __device__ __forceinline__ void wd_average(const V2 x[3], const double h[3], const V2 v[3], double djac,
                                            double* havg, V2* vavg) {  // fe_sw2_wd_average, :40
     double av[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    double factor = wd_wrap<WET>(av, x, h, djac, false,
+    double factor = wd_wrap<STATE>(av, x, h, djac, false,
         [&](double* r) { ig_average(r, djac, h, v); },
         [&](const Cut& c, double* nr) { V2 nv[3]; cut_interp(c, v, nv); ig_average(nr, c.area, c.nh, nv); });
     *havg = 0.; vavg->x = 0.; vavg->y = 0.;
@@ -331,7 +334,7 @@ __device__ __forceinline__ void wd_average(const V2 x[3], const double h[3], con
 }
 
 // fe_sw2_temporal, sw2_body_resid.c:1195
-template <bool WET>
+template <int STATE>
 __device__ __forceinline__ void temporal(double r[9], const V2 x[3], double djac, const double h[3], const V2 v[3],
                                          double wd_fac, double dt_factor, bool add_continuity) {
     double con = dt_factor * wd_fac;
@@ -339,7 +342,7 @@ __device__ __forceinline__ void temporal(double r[9], const V2 x[3], double djac
     double uh[3], vh[3], rx[3] = {0, 0, 0}, ry[3] = {0, 0, 0};
 #pragma unroll
     for (int i = 0; i < 3; i++) { uh[i] = v[i].x * dmax_(h[i], 1e-6); vh[i] = v[i].y * dmax_(h[i], 1e-6); }
-    wd_wrap<WET>(rhs, x, h, djac, true,
+    wd_wrap<STATE>(rhs, x, h, djac, true,
         [&](double* q) { ig_continuity_temporal(q, djac, dt_factor, h); },
         [&](const Cut& c, double* nr) { ig_continuity_temporal(nr, c.area, dt_factor, c.nh); });
     tri_phi_f_lump(djac, con, uh, rx);
@@ -364,9 +367,9 @@ struct TriData {
 };
 
 // fe_sw2_body_resid for a triangle.  PRESSURE is false exactly when the
-// reference perturbs a velocity (sw2_body_resid.c:124-129).  WET (every depth of the three levels is positive) leaves
-// out the cut sub-triangles; what remains is the same operations in the same order.
-template <bool PRESSURE, bool WET>
+// reference perturbs a velocity (sw2_body_resid.c:124-129).  STATE holds at all three levels; ALL_WET and ALL_DRY leave
+// out the cut sub-triangles, and what remains is the same operations in the same order.
+template <bool PRESSURE, int STATE>
 __device__ __forceinline__ void body_resid(const TriData& T, double dt, double alpha, double grav, double r[9]) {
     const V2* x = T.x;
     const V2* g = T.g;
@@ -382,18 +385,18 @@ __device__ __forceinline__ void body_resid(const TriData& T, double dt, double a
 
     double h_wd, oh_wd;
     V2 vel_wd, ovel_wd;
-    wd_average<WET>(x, T.h, T.vel, djac, &h_wd, &vel_wd);
-    wd_average<WET>(x, T.ho, T.velo, djac, &oh_wd, &ovel_wd);
-    double factor = wd_factor<WET>(x, T.h, djac);
-    double factor_old = wd_factor<WET>(x, T.ho, djac);
-    double factor_older = wd_factor<WET>(x, T.hoo, djac);
+    wd_average<STATE>(x, T.h, T.vel, djac, &h_wd, &vel_wd);
+    wd_average<STATE>(x, T.ho, T.velo, djac, &oh_wd, &ovel_wd);
+    double factor = wd_factor<STATE>(x, T.h, djac);
+    double factor_old = wd_factor<STATE>(x, T.ho, djac);
+    double factor_older = wd_factor<STATE>(x, T.hoo, djac);
     double vel_wd_mag = sqrt(vel_wd.x * vel_wd.x + vel_wd.y * vel_wd.y);
     const double roughness = 0.002;   // sw2_body_resid.c:241
 
     {   // advection, :413-434
         double rhs[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
         double c = -1; c *= dt;
-        wd_wrap<WET>(rhs, x, T.h, djac, true,
+        wd_wrap<STATE>(rhs, x, T.h, djac, true,
             [&](double* q) { ig_convection(q, g, djac, c, T.h, T.vel); },
             [&](const Cut& cu, double* nr) { V2 ng[3], nv[3]; cut_grad(cu, ng); cut_interp(cu, T.vel, nv);
                                              ig_convection(nr, ng, cu.area, c, cu.nh, nv); });
@@ -401,9 +404,9 @@ __device__ __forceinline__ void body_resid(const TriData& T, double dt, double a
         for (int i = 0; i < 9; i++) r[i] += rhs[i];
     }
     // temporal, :456-463
-    temporal<WET>(r, x, djac, T.h, T.vel, factor, (1. + alpha / 2.), true);
-    temporal<WET>(r, x, djac, T.ho, T.velo, factor_old, (-1.) * (1. + alpha), T.wd_flag != 2);
-    temporal<WET>(r, x, djac, T.hoo, T.veloo, factor_older, (alpha / 2.), T.wd_flag != 2);
+    temporal<STATE>(r, x, djac, T.h, T.vel, factor, (1. + alpha / 2.), true);
+    temporal<STATE>(r, x, djac, T.ho, T.velo, factor_old, (-1.) * (1. + alpha), T.wd_flag != 2);
+    temporal<STATE>(r, x, djac, T.hoo, T.veloo, factor_older, (alpha / 2.), T.wd_flag != 2);
     // friction, :520-539
     double resistance = roughness / (2.0 * grav);
     {
@@ -423,21 +426,21 @@ __device__ __forceinline__ void body_resid(const TriData& T, double dt, double a
     if (PRESSURE) {   // :710-804
         double rhs[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
         double t1 = -SW2_ONE_2 * grav * dt;
-        wd_wrap<WET>(rhs, x, T.h, djac, true,
+        wd_wrap<STATE>(rhs, x, T.h, djac, true,
             [&](double* q) { ig_pressure(q, g, djac, t1, T.h); },
             [&](const Cut& cu, double* nr) { V2 ng[3]; cut_grad(cu, ng); ig_pressure(nr, ng, cu.area, t1, cu.nh); });
 #pragma unroll
         for (int i = 0; i < 9; i++) r[i] += rhs[i];
         double r2[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
         double t2 = grav * dt;
-        wd_wrap<WET>(r2, x, T.h, djac, true,
+        wd_wrap<STATE>(r2, x, T.h, djac, true,
             [&](double* q) { ig_body_force(q, djac, t2, T.h, grad_z); },
             [&](const Cut& cu, double* nr) { ig_body_force(nr, cu.area, t2, cu.nh, grad_z); });
 #pragma unroll
         for (int i = 0; i < 9; i++) r[i] += r2[i];
         double r3[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
         double t3 = SW2_ONE_2 * dt * grav;
-        wd_wrap<WET>(r3, x, T.h, djac, true,
+        wd_wrap<STATE>(r3, x, T.h, djac, true,
             [&](double* q) { ig_boundary_pressure(q, x, t3, T.h); },
             [&](const Cut& cu, double* nr) { ig_boundary_pressure(nr, cu.nx, t3, cu.nh); });
 #pragma unroll
@@ -455,17 +458,17 @@ __device__ __forceinline__ void body_resid(const TriData& T, double dt, double a
         double sr = sqrt(vel_wd.x * vel_wd.x + vel_wd.y * vel_wd.y + cel2 + SW2_SMALL);
         double tau = 0.5 * le / sr;
         double dfdt[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-        wd_wrap<WET>(dfdt, x, T.ho, djac, false,
+        wd_wrap<STATE>(dfdt, x, T.ho, djac, false,
             [&](double* q) { ig_average(q, djac, T.ho, T.velo); },
             [&](const Cut& cu, double* nr) { V2 nv[3]; cut_interp(cu, T.velo, nv); ig_average(nr, cu.area, cu.nh, nv); });
         double dudt = -dfdt[1], dvdt = -dfdt[2], dhdt = -dfdt[0];
         double dfn[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-        wd_wrap<WET>(dfn, x, T.h, djac, false,
+        wd_wrap<STATE>(dfn, x, T.h, djac, false,
             [&](double* q) { ig_average(q, djac, T.h, T.vel); },
             [&](const Cut& cu, double* nr) { V2 nv[3]; cut_interp(cu, T.vel, nv); ig_average(nr, cu.area, cu.nh, nv); });
         dudt += dfn[1]; dvdt += dfn[2]; dhdt += dfn[0];
         double adv[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-        double fac = wd_wrap<WET>(adv, x, T.h, djac, false,
+        double fac = wd_wrap<STATE>(adv, x, T.h, djac, false,
             [&](double* q) { ig_gls_convection(q, g, djac, dt, 1, T.h, T.vel); },
             [&](const Cut& cu, double* nr) { V2 ng[3], nv[3]; double nf[3]; cut_grad(cu, ng); cut_interp(cu, T.vel, nv);
                                              cut_interp(cu, T.h, nf); ig_gls_convection(nr, ng, cu.area, dt, 1, nf, nv); });

@@ -47,12 +47,20 @@ __device__ __forceinline__ bool all_wet(const TriData& T, double margin) {
     for (int a = 0; a < 3; a++) w = w && T.h[a] > margin && T.ho[a] > 0.0 && T.hoo[a] > 0.0;
     return w;
 }
+// no depth positive, at the current level none above -margin
+__device__ __forceinline__ bool all_dry(const TriData& T, double margin) {
+    bool d = true;
+#pragma unroll
+    for (int a = 0; a < 3; a++) d = d && T.h[a] <= -margin && T.ho[a] <= 0.0 && T.hoo[a] <= 0.0;
+    return d;
+}
 // What bounds the element kernels is latency: 1600 instructions a residual, most of them FP64 in long chains (13
 // divisions, 6 square roots), at few warps an SM.  Elements that are wet at all levels, most of them, take a
 // branch without the cut sub-triangles' code (~1000 operations left), and kElemBlocks CTAs an SM, 168 registers,
 // is the best of 2 to 5 for the two branches together (FD Jacobian of 1M wet triangles: 1.43, 1.29, 1.49, 1.75 ms; 2.42 ms
 // with the general code for all, at 254 registers).  Kernels of their own for the wet and the cut elements pay the loads
-// twice (1.80 ms).
+// twice (1.80 ms).  The general code spills there (k_resid 160 bytes read back, k_fd_tri 1000 to 1400), which costs less than
+// the third CTA gives; where it costs more, on dry land and on small meshes, see k_fd_tri.
 // Neighbouring elements stay in neighbouring blocks: spreading the cut ones over the grid mixes the two branches' code in
 // every SM's instruction cache (FD Jacobian of a 250k-triangle beach 0.64 -> 0.87 ms).
 constexpr int kElemThreads = 128, kElemBlocks = 3;
@@ -105,6 +113,7 @@ __global__ void k_dry_mask(int nnodes, const double* __restrict__ sol_old, int* 
 // Every triangle of the warp is wet: one cut triangle takes its whole warp through the general code, which gives wet ones the
 // same bits.  With a choice per triangle such a warp ran both: 30.2 us, now 27.3, for the residual of the 576-node basin drying out.
 __device__ __forceinline__ bool warp_wet(const TriData& T, double least) { return __all_sync(__activemask(), all_wet(T, least)); }
+__device__ __forceinline__ bool warp_dry(const TriData& T, double least) { return __all_sync(__activemask(), all_dry(T, least)); }
 
 // ---------------------------------------------------------------- residuals
 __device__ __forceinline__ void seg_residual(const MeshView& M, const StepParams& P, const double* __restrict__ sol, int s,
@@ -123,8 +132,8 @@ __global__ void __launch_bounds__(kElemThreads, kElemBlocks) k_resid(MeshView M,
     TriData T;
     load_tri(M, sol, sol_old, sol_older, wd_flag, e, T);
     double r[9];
-    if (warp_wet(T, 0.0)) body_resid<true, true>(T, P.dt, P.alpha, P.grav, r);
-    else body_resid<true, false>(T, P.dt, P.alpha, P.grav, r);
+    if (warp_wet(T, 0.0)) body_resid<true, ALL_WET>(T, P.dt, P.alpha, P.grav, r);
+    else body_resid<true, ANY>(T, P.dt, P.alpha, P.grav, r);
     double* out = ER + 9 * (size_t)e;
 #pragma unroll
     for (int i = 0; i < 9; i++) out[i] = r[i];
@@ -162,7 +171,8 @@ __global__ void k_gather_resid(int nnodes, AssemblyMaps A, const double* __restr
 // column (node i, var k) = (R(u + eps e) - R(u - eps e)) / (2 eps).
 // Template VAR: 0 perturbs h (pressure terms evaluated), 1/2 perturb u/v
 // (pressure terms skipped, as the reference's PRESSURE_FLAG does).
-template <int VAR, bool WET>
+// TOGETHER: 2 lets the two signs overlap, 1 evaluates them in turn by the same code.
+template <int VAR, int STATE, int TOGETHER>
 __device__ __forceinline__ void fd_column(const TriData& T, const StepParams& P, int i, double* __restrict__ out) {
     double u0 = VAR == 0 ? (i == 0 ? T.h[0] : i == 1 ? T.h[1] : T.h[2])
               : VAR == 1 ? (i == 0 ? T.vel[0].x : i == 1 ? T.vel[1].x : T.vel[2].x)
@@ -170,7 +180,7 @@ __device__ __forceinline__ void fd_column(const TriData& T, const StepParams& P,
     const double eps = fd_eps(u0);
     const double eps2 = 2.0 * eps;
     double Rp[9], Rm[9];
-#pragma unroll
+#pragma unroll TOGETHER
     for (int sgn = 0; sgn < 2; sgn++) {
         TriData Q = T;
         const double d = (sgn == 0 ? 1 : -1) * eps;
@@ -181,13 +191,24 @@ __device__ __forceinline__ void fd_column(const TriData& T, const StepParams& P,
             else if (VAR == 1) Q.vel[a].x += d;
             else Q.vel[a].y += d;
         }
-        body_resid<VAR == 0, WET>(Q, P.dt, P.alpha, P.grav, sgn == 0 ? Rp : Rm);
+        body_resid<VAR == 0, STATE>(Q, P.dt, P.alpha, P.grav, Rm);
+        if (sgn == 0) {
+#pragma unroll
+            for (int r = 0; r < 9; r++) Rp[r] = Rm[r];
+        }
     }
 #pragma unroll
     for (int r = 0; r < 9; r++) out[r] = (Rp[r] - Rm[r]) / eps2;
 }
-template <int VAR>
-__global__ void __launch_bounds__(kElemThreads, kElemBlocks) k_fd_tri(MeshView M, StepParams P, const double* __restrict__ sol,
+// Three branches, chosen by warp: wet, dry (a warp of dry land needs no sub-triangle either) and the general one.
+// BLOCKS CTAs an SM: kElemBlocks, and 2 (254 registers, no spills) where they hold the whole grid, since a third CTA then
+// brings nothing (FD Jacobian of 1058 cut triangles 176 us with 3, 154 with 2).  The signs follow one another, so that
+// the three branches fit the instruction cache together: where wet and general warps mix, both fetch their code anew
+// (1M triangles, 0.5 % of the nodes dry here and there: 12.6 ms with the signs overlapped, 9.4 now; wet 1.29, now 1.21; the
+// land dry 2.16, now 0.81; beach of 1M triangles 1.85, now 1.61).  The general code of the small grids overlaps them, for
+// its latency.  With general code alone for everything these were 12.0, 2.42, 1.73, 2.91 ms, and 146 us for the cut 1058.
+template <int VAR, int BLOCKS>
+__global__ void __launch_bounds__(kElemThreads, BLOCKS) k_fd_tri(MeshView M, StepParams P, const double* __restrict__ sol,
                                                 const double* __restrict__ sol_old, const double* __restrict__ sol_older,
                                                 const int* __restrict__ wd_flag, double* __restrict__ EJ, int Etot) {
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
@@ -196,9 +217,11 @@ __global__ void __launch_bounds__(kElemThreads, kElemBlocks) k_fd_tri(MeshView M
     TriData T;
     load_tri(M, sol, sol_old, sol_older, wd_flag, e, T);
     double* out = EJ + ((size_t)(i * 3 + VAR) * Etot + e) * 9;
-    // a depth above 2e-4 stays positive under its perturbation (fd_eps: at most 1e-4, or 1e-4 of it)
-    if (warp_wet(T, VAR == 0 ? 2e-4 : 0.0)) fd_column<VAR, true>(T, P, i, out);
-    else fd_column<VAR, false>(T, P, i, out);
+    // a depth above 2e-4 stays positive under its perturbation, one below -2e-4 negative (fd_eps: at most 1e-4, or 1e-4 of it)
+    const double least = VAR == 0 ? 2e-4 : 0.0;
+    if (warp_wet(T, least)) fd_column<VAR, ALL_WET, 1>(T, P, i, out);
+    else if (warp_dry(T, least)) fd_column<VAR, ALL_DRY, 1>(T, P, i, out);
+    else fd_column<VAR, ANY, BLOCKS == kElemBlocks ? 1 : 2>(T, P, i, out);
 }
 
 __global__ void k_fd_seg(MeshView M, StepParams P, const double* __restrict__ sol, double* __restrict__ EJ, int Etot) {
@@ -394,9 +417,16 @@ void launch_elem_jac(const MeshView& M, const StepParams& P, const double* sol, 
     const int Etot = M.ntri + M.nseg;
     if (M.ntri) {
         dim3 g(blocks(M.ntri, kElemThreads), 3);
-        k_fd_tri<0><<<g, kElemThreads, 0, st>>>(M, P, sol, sol_old, sol_older, wd_flag, EJ, Etot);
-        k_fd_tri<1><<<g, kElemThreads, 0, st>>>(M, P, sol, sol_old, sol_older, wd_flag, EJ, Etot);
-        k_fd_tri<2><<<g, kElemThreads, 0, st>>>(M, P, sol, sol_old, sol_older, wd_flag, EJ, Etot);
+        int dev = 0, sms = 148;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        auto run = [&](auto by_h, auto by_u, auto by_v) {
+            by_h<<<g, kElemThreads, 0, st>>>(M, P, sol, sol_old, sol_older, wd_flag, EJ, Etot);
+            by_u<<<g, kElemThreads, 0, st>>>(M, P, sol, sol_old, sol_older, wd_flag, EJ, Etot);
+            by_v<<<g, kElemThreads, 0, st>>>(M, P, sol, sol_old, sol_older, wd_flag, EJ, Etot);
+        };
+        if ((long)g.x * g.y <= 2L * sms) run(k_fd_tri<0, 2>, k_fd_tri<1, 2>, k_fd_tri<2, 2>);
+        else run(k_fd_tri<0, kElemBlocks>, k_fd_tri<1, kElemBlocks>, k_fd_tri<2, kElemBlocks>);
     }
     if (M.nseg) {
         dim3 g(blocks(M.nseg, 128), 6);
