@@ -63,7 +63,7 @@ __device__ __forceinline__ double block_max(double v, double* sh) {
     return t;
 }
 // Publish this block's partials; returns true in warp 0 of the last block, whose lanes then
-// reduce every block's partials (part_sum, part_max).
+// reduce every block's partials (parts).
 __device__ __forceinline__ bool last_block(Reduce R, const double* vals, int nv) {
     __shared__ bool is_last;
     if (threadIdx.x == 0) {
@@ -75,8 +75,8 @@ __device__ __forceinline__ bool last_block(Reduce R, const double* vals, int nv)
     __syncthreads();
     return is_last && threadIdx.x < 32;
 }
-__device__ __forceinline__ double part_sum(const Reduce& R, int i) { return ordered_sum(R.partial + i, 4, (int)gridDim.x); }
-__device__ __forceinline__ double part_max(const Reduce& R, int i) { return warp_max(R.partial + i, 4, (int)gridDim.x); }
+template <unsigned MAXES, int N>
+__device__ __forceinline__ void parts(const Reduce& R, double (&out)[N]) { reduce_partials<MAXES>(R.partial, (int)gridDim.x, out); }
 
 // ---------------------------------------------------------------- Newton norms
 __global__ void __launch_bounds__(256) k_norms(int n, const double* __restrict__ res, const double* __restrict__ dsol,
@@ -93,7 +93,9 @@ __global__ void __launch_bounds__(256) k_norms(int n, const double* __restrict__
     double v[3];
     v[0] = block_max<256>(mx, sh); v[1] = block_sum<256>(l2, sh); v[2] = block_max<256>(im, sh);
     if (last_block(R, v, 3)) {
-        const double a = part_max(R, 0), b = part_sum(R, 1), c = part_max(R, 2);
+        double t[3];
+        parts<5>(R, t);
+        const double a = t[0], b = t[1], c = t[2];
         if (threadIdx.x == 0) { R.out[0] = a; R.out[1] = b; R.out[2] = c; }
     }
 }
@@ -276,7 +278,9 @@ __global__ void __launch_bounds__(256) k_bicg_init2(BlockCSR A, KrylovVecs<VT> V
     double v[3];
     v[0] = block_max<256>(rmax, sh); v[1] = block_max<256>(bmax, sh); v[2] = block_sum<256>(rr, sh);
     if (last_block(R, v, 3)) {
-        const double a = part_max(R, 0), b = part_max(R, 1), c = part_sum(R, 2);
+        double t[3];
+        parts<3>(R, t);
+        const double a = t[0], b = t[1], c = t[2];
         if (threadIdx.x) return;
         S->rnorm = a; S->bnorm = b; S->rho = c;
         S->rhop = 1.0; S->alpha = 1.0; S->omega = 1.0; S->beta = 0.0; S->it = 0; S->status = 0;
@@ -307,7 +311,9 @@ __global__ void __launch_bounds__(256) k_bicg_spmv_p(BlockCSR A, KrylovVecs<VT> 
     double v[1];
     v[0] = block_sum<256>(qa, sh);
     if (last_block(R, v, 1)) {
-        const double g = part_sum(R, 0);
+        double t[1];
+        parts<0>(R, t);
+        const double g = t[0];
         if (threadIdx.x) return;
         S->gamma = g;
         if (g == 0.0 || !isfinite(g)) { S->status = 1; S->done = 1; }
@@ -350,7 +356,9 @@ __global__ void __launch_bounds__(256) k_bicg_spmv_s(BlockCSR A, KrylovVecs<VT> 
     double v[3];
     v[0] = block_sum<256>(ss, sh); v[1] = block_sum<256>(aa, sh); v[2] = block_sum<256>(aq, sh);
     if (last_block(R, v, 3)) {
-        const double a = part_sum(R, 0), b = part_sum(R, 1), c = part_sum(R, 2);
+        double t[3];
+        parts<0>(R, t);
+        const double a = t[0], b = t[1], c = t[2];
         if (threadIdx.x) return;
         if (b == 0.0) {            // s == 0: x + alpha p is the solution
             S->omega = 0.0; S->status = 3;
@@ -390,7 +398,9 @@ __global__ void __launch_bounds__(256) k_bicg_update(int n, KrylovVecs<VT> V, Kr
     double v[1];
     v[0] = block_max<256>(rmax, sh);
     if (last_block(R, v, 1)) {
-        const double m = part_max(R, 0);
+        double t[1];
+        parts<1>(R, t);
+        const double m = t[0];
         if (threadIdx.x) return;
         S->rnorm = m;
         S->it += 1;
@@ -463,7 +473,9 @@ __global__ void __launch_bounds__(256) k_resid_pnorm(BlockCSR A, const double* _
     double v[1];
     v[0] = block_max<256>(zmax, sh);
     if (last_block(R, v, 1)) {
-        const double mm = part_max(R, 0);
+        double t[1];
+        parts<1>(R, t);
+        const double mm = t[0];
         if (threadIdx.x == 0) R.out[0] = mm;
     }
 }
@@ -610,7 +622,9 @@ __global__ void __launch_bounds__(256) k_bicg_init_pc(int n, KrylovVecs<VT> V, K
     double v[3];
     v[0] = block_max<256>(rmax, sh); v[1] = block_max<256>(bmax, sh); v[2] = block_sum<256>(rr, sh);
     if (last_block(R, v, 3)) {
-        const double a = part_max(R, 0), b = part_max(R, 1), c = part_sum(R, 2);
+        double t[3];
+        parts<3>(R, t);
+        const double a = t[0], b = t[1], c = t[2];
         if (threadIdx.x) return;
         S->rnorm = a; S->bnorm = b; S->rho = c;
         S->rhop = 1.0; S->alpha = 1.0; S->omega = 1.0; S->beta = 0.0; S->it = 0; S->status = 0;
@@ -630,7 +644,9 @@ __global__ void __launch_bounds__(256) k_bicg_alpha(int n, KrylovVecs<VT> V, Kry
     double v[1];
     v[0] = block_sum<256>(qa, sh);
     if (last_block(R, v, 1)) {
-        const double g = part_sum(R, 0);
+        double t[1];
+        parts<0>(R, t);
+        const double g = t[0];
         if (threadIdx.x) return;
         S->gamma = g;
         if (g == 0.0 || !isfinite(g)) { S->status = 1; S->done = 1; }
@@ -651,7 +667,9 @@ __global__ void __launch_bounds__(256) k_bicg_omega(int n, KrylovVecs<VT> V, Kry
     double v[3];
     v[0] = block_sum<256>(ss, sh); v[1] = block_sum<256>(aa, sh); v[2] = block_sum<256>(aq, sh);
     if (last_block(R, v, 3)) {
-        const double a = part_sum(R, 0), b = part_sum(R, 1), c = part_sum(R, 2);
+        double t[3];
+        parts<0>(R, t);
+        const double a = t[0], b = t[1], c = t[2];
         if (threadIdx.x) return;
         if (b == 0.0) { S->omega = 0.0; S->status = 3; }
         else {
@@ -834,7 +852,9 @@ __global__ void __launch_bounds__(256) k_maxabs(int n, const double* __restrict_
     double v[2];
     v[0] = block_max<256>(m, sh); v[1] = block_max<256>(bad, sh);
     if (last_block(R, v, 2)) {
-        const double a = part_max(R, 0), b = part_max(R, 1);
+        double t[2];
+        parts<3>(R, t);
+        const double a = t[0], b = t[1];
         if (threadIdx.x) return;
         R.out[0] = b > 0 ? NAN : a;   // a non-finite entry is reported, not hidden by fmax
     }
@@ -850,7 +870,9 @@ __global__ void __launch_bounds__(256) k_maxabs_unscaled(int n, const double* __
     double v[2];
     v[0] = block_max<256>(m, sh); v[1] = block_max<256>(bad, sh);
     if (last_block(R, v, 2)) {
-        const double a = part_max(R, 0), b = part_max(R, 1);
+        double t[2];
+        parts<3>(R, t);
+        const double a = t[0], b = t[1];
         if (threadIdx.x) return;
         R.out[0] = b > 0 ? NAN : a;
     }

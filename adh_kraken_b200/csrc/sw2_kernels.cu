@@ -382,8 +382,9 @@ __global__ void __launch_bounds__(256) k_mass_balance(MeshView M, const double* 
     }
     __syncthreads();
     if (is_last && threadIdx.x < 32) {
-        const double a = ordered_sum(partial, 4, (int)gridDim.x), b = ordered_sum(partial + 1, 4, (int)gridDim.x);
-        if (threadIdx.x == 0) { out[0] = a * density; out[1] = b; }
+        double t[2];
+        reduce_partials<0>(partial, (int)gridDim.x, t);
+        if (threadIdx.x == 0) { out[0] = t[0] * density; out[1] = t[1]; }
     }
 }
 
