@@ -16,6 +16,7 @@
 #include <vector>
 #include <algorithm>
 #include <string>
+#include <sys/mman.h>
 #include "../../include/adh_sw2_gpu.h"
 #include "sw2_launch.h"
 
@@ -45,6 +46,7 @@ extern "C" const char* sw2g_last_error(void) { return g_err.c_str(); }
 
 static const int kChunk = 8;   // BiCGStab iterations per graph replay
 static const int kSmallChunk = 256;   // BiCGStab iterations per launch of the small meshes' solver
+static const int kStageSlots = 16;   // pieces in the ring of large downloads
 static const double kPatchTileEdges = 7.0;   // tile side of the AMG chunk corrections, in mean edge lengths
 
 struct ProfRec { int cls; cudaEvent_t a, b; };
@@ -101,8 +103,9 @@ struct sw2g_model {
     double *d_partial = nullptr, *d_rout = nullptr; unsigned int* d_counter = nullptr;
     KrylovScalars* d_ks = nullptr;
     double* h_rout = nullptr; KrylovScalars* h_ks = nullptr; int* h_state = nullptr;   // pinned
-    char* h_stage = nullptr;           // pinned ring of large downloads (models whose matrix is one), kStageSlots pieces
-    std::vector<cudaEvent_t> stage_ev;
+    char* h_stage = nullptr;           // pinned ring of large downloads (download), kStageSlots pieces, and their copies' events
+    cudaEvent_t stage_ev[kStageSlots] = {};
+    bool stage_tried = false;
     cudaGraphExec_t graph64[3] = {nullptr, nullptr, nullptr}, graph32[3] = {nullptr, nullptr, nullptr};   // [precond]
     // multicolour block ILU(0)
     std::vector<int> h_color_ptr;
@@ -168,28 +171,57 @@ static int upload(sw2g_model* m, T** p, const T* h, size_t count) {
 // triangles.  Pieces go to a pinned ring instead, from where a few threads copy them on, so that PCIe, the copies and
 // the page faults of several cores overlap.  The threads live for the call; without them (or without the ring) the plain
 // copy is made.  Destinations that are pinned already are copied to directly.  Complete on return.
+// assemble_jacobian with the plain copy and here, into a fresh array and into one used before (ms): 8.2 MB 4.3, 1.7 and 0.78,
+// 0.61; 14 MB 7.2, 2.6 and 1.20, 1.05; 65 MB 32.8, 10.2 and 4.7, 3.2.  Below the line a used array gains nothing (6.2 MB: 0.63
+// plain, 0.55 to 0.94 here, by how soon the threads run).  The first round of the ring is queued before the threads start:
+// after them, arrays of 8 to 20 MB took up to 1.4 times the plain copy.
 static const size_t kStageMin = 8u << 20, kStagePiece = 1u << 20;
-static const int kStageSlots = 16, kStageThreads = 8;
+static const int kStageThreads = 8;
+// The ring, pinned by the first large download, so that models without one do not pay for it.  Huge pages where the system
+// gives them: 16 MB are pinned in 1.8 ms then, in 14 to 16 as small pages.
+static bool stage_ring(sw2g_model* m) {
+    if (m->h_stage || m->stage_tried) return m->h_stage != nullptr;
+    m->stage_tried = true;
+    const size_t huge = 2u << 20, bytes = (kStageSlots * kStagePiece + huge - 1) / huge * huge;
+    void* p = aligned_alloc(huge, bytes);
+    if (!p) return false;
+    madvise(p, bytes, MADV_HUGEPAGE);
+    if (cudaHostRegister(p, bytes, cudaHostRegisterDefault) != cudaSuccess) { cudaGetLastError(); free(p); return false; }
+    for (cudaEvent_t& e : m->stage_ev)
+        if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
+            cudaGetLastError();
+            cudaHostUnregister(p);
+            free(p);
+            return false;
+        }
+    m->h_stage = (char*)p;
+    return true;
+}
 static int download(sw2g_model* m, void* dst, const void* src, size_t bytes) {
-    cudaPointerAttributes at{};
-    bool plain = bytes < kStageMin || !m->h_stage;
-    if (!plain) {
-        if (cudaPointerGetAttributes(&at, dst) != cudaSuccess) cudaGetLastError();
-        else plain = at.type != cudaMemoryTypeUnregistered;
-    }
-    const unsigned cores = std::thread::hardware_concurrency();
-    const int nt = (int)std::min<unsigned>(kStageThreads, cores ? cores : 1);
-    if (plain || nt < 2) {
+    auto plain = [&]() -> int {
         CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, m->st));
         CK(cudaStreamSynchronize(m->st));
         return SW2G_OK;
-    }
+    };
+    cudaPointerAttributes at{};
+    if (bytes < kStageMin) return plain();
+    if (cudaPointerGetAttributes(&at, dst) != cudaSuccess) cudaGetLastError();
+    else if (at.type != cudaMemoryTypeUnregistered) return plain();
+    const unsigned cores = std::thread::hardware_concurrency();
+    const int nt = (int)std::min<unsigned>(kStageThreads, cores);
+    if (nt < 2 || !stage_ring(m)) return plain();
     const long pieces = (long)((bytes + kStagePiece - 1) / kStagePiece);
     std::mutex mu;
     std::condition_variable cv;
     long issued = 0;                       // pieces whose copy to the ring is in the stream
-    std::vector<char> done(pieces, 0);     // pieces copied on
+    std::vector<char> done;                // pieces copied on
     cudaError_t err = cudaSuccess;         // the first failure; everyone stops
+    auto queue = [&](long k) {             // piece k into its slot of the ring
+        const int slot = (int)(k % kStageSlots);
+        const cudaError_t e = cudaMemcpyAsync(m->h_stage + slot * kStagePiece, (const char*)src + k * kStagePiece,
+                                              std::min(kStagePiece, bytes - k * kStagePiece), cudaMemcpyDeviceToHost, m->st);
+        return e != cudaSuccess ? e : cudaEventRecord(m->stage_ev[slot], m->st);
+    };
     auto work = [&](int w) {
         cudaSetDevice(m->device);
         for (long k = w; k < pieces; k += nt) {
@@ -208,31 +240,29 @@ static int download(sw2g_model* m, void* dst, const void* src, size_t bytes) {
             cv.notify_all();
         }
     };
+    // the first round of the ring is on its way while the threads start
+    for (; issued < std::min<long>(pieces, kStageSlots); issued++) CK(queue(issued));
     std::vector<std::thread> team;
     try {
+        done.assign(pieces, 0);
         team.reserve(nt);
         for (int w = 0; w < nt; w++) team.emplace_back(work, w);
-    } catch (...) {   // no (more) threads: stop those that started and copy plainly
+    } catch (...) {   // no memory or no (more) threads: stop those that started and copy plainly
         {
             std::lock_guard<std::mutex> lock(mu);
             err = cudaErrorUnknown;
             cv.notify_all();
         }
         for (std::thread& t : team) t.join();
-        CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, m->st));
-        CK(cudaStreamSynchronize(m->st));
-        return SW2G_OK;
+        return plain();
     }
-    for (long k = 0; k < pieces; k++) {
-        if (k >= kStageSlots) {            // the slot's last piece has left it
+    for (long k = issued; k < pieces; k++) {
+        {                                  // the slot's last piece has left it
             std::unique_lock<std::mutex> lock(mu);
             cv.wait(lock, [&] { return done[k - kStageSlots] || err != cudaSuccess; });
             if (err != cudaSuccess) break;
         }
-        const int slot = (int)(k % kStageSlots);
-        cudaError_t e = cudaMemcpyAsync(m->h_stage + slot * kStagePiece, (const char*)src + k * kStagePiece,
-                                        std::min(kStagePiece, bytes - k * kStagePiece), cudaMemcpyDeviceToHost, m->st);
-        if (e == cudaSuccess) e = cudaEventRecord(m->stage_ev[slot], m->st);
+        const cudaError_t e = queue(k);
         std::lock_guard<std::mutex> lock(mu);
         if (e != cudaSuccess && err == cudaSuccess) err = e;
         issued = k + 1;
@@ -536,16 +566,6 @@ extern "C" int sw2g_create(const sw2g_mesh* mesh, void* cuda_stream, sw2g_model*
             if (r != SW2G_OK) return fail(r);
         }
     }
-    if (sizeof(double) * (size_t)m->nnz >= kStageMin) {   // without the ring large downloads are plain copies
-        if (cudaMallocHost((void**)&m->h_stage, kStageSlots * kStagePiece) != cudaSuccess) { cudaGetLastError(); m->h_stage = nullptr; }
-        for (int k = 0; m->h_stage && k < kStageSlots; k++) {
-            cudaEvent_t e;
-            if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess) { m->stage_ev.push_back(e); continue; }
-            cudaGetLastError();
-            cudaFreeHost(m->h_stage);
-            m->h_stage = nullptr;
-        }
-    }
     m->M = MeshView{V, T, S, m->d_tri, m->d_ex, m->d_ey, m->d_ez, m->d_gx, m->d_gy, m->d_djac,
                     m->d_seg, m->d_snx, m->d_sny, m->d_sdjac, m->d_skind, m->d_sz0};
     m->A = AssemblyMaps{m->nslots, m->d_rptr, m->d_rmap, m->d_jptr, m->d_jmap, m->d_boff, m->d_blen};
@@ -579,8 +599,9 @@ extern "C" void sw2g_destroy(sw2g_model* m) {
     if (m->h_rout) cudaFreeHost(m->h_rout);
     if (m->h_ks) cudaFreeHost(m->h_ks);
     if (m->h_state) cudaFreeHost(m->h_state);
-    if (m->h_stage) cudaFreeHost(m->h_stage);
-    for (cudaEvent_t e : m->stage_ev) cudaEventDestroy(e);
+    if (m->h_stage) { cudaHostUnregister(m->h_stage); free(m->h_stage); }
+    for (cudaEvent_t e : m->stage_ev)
+        if (e) cudaEventDestroy(e);
     if (m->h_pflag) cudaFreeHost(m->h_pflag);
     if (m->h_cptr) cudaFreeHost(m->h_cptr);
     if (m->h_cown) cudaFreeHost(m->h_cown);
