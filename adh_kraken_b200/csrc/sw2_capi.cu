@@ -87,7 +87,8 @@ struct sw2g_model {
     double *d_sol = nullptr, *d_sol_old = nullptr, *d_sol_older = nullptr, *d_dirichlet = nullptr, *d_guess = nullptr;
     int *d_bc_mask = nullptr, *d_mask_save = nullptr;
     bool guess_set = false;
-    SmallPlan small;         // the small meshes' Krylov solver
+    SmallPlan small;         // the small meshes' Krylov solver (small_setup)
+    bool small_tried = false;
     std::vector<int> small_order;   // its order of the nodes
     int small_m32 = 0, small_pc32 = 0;   // restart length and preconditioner of its last FP32 GMRES cycle
     bool can_undo = false;   // the levels were rotated by the last sw2g_step
@@ -346,6 +347,21 @@ static int small_level(sw2g_model* m, int l, const std::vector<int>& bptr, const
     return SW2G_OK;
 }
 
+// The small meshes' solver, on the first set-up of a preconditioner that it takes (0.6 to 1 ms, which models that only
+// assemble do not pay)
+static int small_setup(sw2g_model* m) {
+    if (m->small_tried || m->V > kClusterNodes) return SW2G_OK;
+    m->small_tried = true;
+    int limit = 0;
+    if (cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, m->device) != cudaSuccess) cudaGetLastError();
+    m->small = small_solver_plan(limit);
+    if (m->small.ctas == 0) return SW2G_OK;
+    m->small_order = small_order(m->h_bptr, m->h_bcol, m->V, m->small.ctas);
+    const int r = small_level(m, 0, m->h_bptr, m->h_bcol, m->small_order);
+    if (r != SW2G_OK) m->small.ctas = 0;
+    return r;
+}
+
 extern "C" void sw2g_default_opts(sw2g_newton_opts* o) {
     o->tol_nonlin = 1e-8; o->inc_nonlin = 1e-6; o->max_nonlin_it = 10; o->max_linesearch_cuts = 5;
     o->krylov_max_it = 4000; o->krylov_tol = 1e-11; o->krylov_precision = 64;
@@ -556,16 +572,6 @@ extern "C" int sw2g_create(const sw2g_mesh* mesh, void* cuda_stream, sw2g_model*
         cudaMallocHost((void**)&m->h_state, sizeof(int)) != cudaSuccess) {
         g_err = "cudaMallocHost failed"; return fail(SW2G_ERR_NOMEM);
     }
-    if (V <= kClusterNodes) {
-        int limit = 0;
-        if (cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, m->device) != cudaSuccess) cudaGetLastError();
-        m->small = small_solver_plan(limit);
-        if (m->small.ctas > 0) {
-            m->small_order = small_order(m->h_bptr, m->h_bcol, V, m->small.ctas);
-            const int r = small_level(m, 0, m->h_bptr, m->h_bcol, m->small_order);
-            if (r != SW2G_OK) return fail(r);
-        }
-    }
     m->M = MeshView{V, T, S, m->d_tri, m->d_ex, m->d_ey, m->d_ez, m->d_gx, m->d_gy, m->d_djac,
                     m->d_seg, m->d_snx, m->d_sny, m->d_sdjac, m->d_skind, m->d_sz0};
     m->A = AssemblyMaps{m->nslots, m->d_rptr, m->d_rmap, m->d_jptr, m->d_jmap, m->d_boff, m->d_blen};
@@ -720,6 +726,7 @@ static int do_precond_setup(sw2g_model* m, const double* vals, int precond, int 
         return build_patches(m, vals);
     }
     if (precond == SW2G_PC_BILU0) {
+        TRY(small_setup(m));
         ProfScope ps(m, 3, 1 + m->ilu.ncolors);
         launch_bilu_factor(m->B, m->ilu, vals, m->d_lu, m->d_inv, m->st);
     } else {
@@ -758,6 +765,7 @@ static int aggregate_nodes(int n, const std::vector<int>& gp, const std::vector<
 }
 
 static int build_amg(sw2g_model* m) {
+    TRY(small_setup(m));               // (its plan of the levels is made below)
     struct HostLev { int n; std::vector<int> bptr, bcol, dpos; };
     struct HostLink { std::vector<int> agg, mptr, mem, gptr, gsrc; };
     std::vector<HostLev> L(1);
