@@ -161,6 +161,20 @@ def start_cpu_reference(nsteps_total):
     return case, refio.HarnessRun("run", case, extra=(nsteps_total,))
 
 
+def cpu_baseline_failed(e):
+    """What the bench line says of a baseline that could not be started or finished: reported, not fatal."""
+    return {"value": None, "unit": UNIT, "cores": 1, "kind": "reference", "sample": f"failed: {e}"}
+
+
+def begin_cpu_baseline(nsteps_total):
+    """((case, run) of the reference started in the background, None), or (None, what the bench line reports)
+    where it cannot be started, as without its harness."""
+    try:
+        return start_cpu_reference(nsteps_total), None
+    except Exception as e:  # noqa: BLE001
+        return None, cpu_baseline_failed(e)
+
+
 def cpu_reference_result(run, case, skip):
     rec = run.wait(timeout=3600)
     secs = np.asarray(rec["step_seconds"], dtype=np.float64)
@@ -223,9 +237,9 @@ def run_ours(args, world, rank, local, dist):
 
     torch.cuda.set_device(local)
     K, W = args.steps, args.warmup
-    cpu_run = None
+    cpu_run, cpu = None, None
     if rank == 0 and world == 1 and not args.no_cpu_baseline and args.workload == "beach4M":
-        cpu_run = start_cpu_reference(W + K)    # CPU work in the background while the GPU runs
+        cpu_run, cpu = begin_cpu_baseline(W + K)    # CPU work in the background while the GPU runs
     if args.workload == "basin1M":
         from adh_kraken_b200.mesh import basin_case
         case = basin_case(n=707, seed=2, nsteps=W + 2 * K + 8)
@@ -429,7 +443,7 @@ def run_ours(args, world, rank, local, dist):
 
     # the reference's CPU run on the sample (rank 0): timing and the final state, and our two
     # paths on the same sample with the same options, compared with it
-    cpu, sample_err = None, None
+    sample_err = None
     if cpu_run is not None:
         try:
             scase, srun = cpu_run
@@ -447,8 +461,8 @@ def run_ours(args, world, rank, local, dist):
                 sample_err["steps"] = W + K
                 sample_err["note"] = ("state after the same steps as the reference's run; the reference applies "
                                       "its absolute Newton test 1e-8, ours the relative one")
-        except Exception as e:  # noqa: BLE001 - reported, not fatal
-            cpu = {"value": None, "unit": UNIT, "cores": 1, "kind": "reference", "sample": f"failed: {e}"}
+        except Exception as e:  # noqa: BLE001
+            cpu = cpu_baseline_failed(e)
 
     if rank != 0:
         _cleanup(fast, plain, guesser)
