@@ -1995,15 +1995,19 @@ extern "C" int sw2g_time_kernel(sw2g_model* m, int which, int reps, double* avg_
     CK(cudaEventElapsedTime(&ms, a, b));
     m->ev_pool.push_back(a); m->ev_pool.push_back(b);
     *avg_ms = ms / reps;
+    // What a matrix pass over level 0 cannot do without, in values of b bytes: the values, a column per 3x3 block and a pointer
+    // per node; x and y; a smoothing sweep also the blocks of the smoother and the right-hand side
+    auto product = [&](double b) { return b * nnz + 4.0 * nnz / 9.0 + 4.0 * m->V + 2.0 * b * n; };
+    auto sweep = [&](double b) { return product(b) + 9.0 * b * m->V + b * n; };
     switch (which) {   // algorithmic bytes of one launch
-        case 0: *bytes = 12.0 * nnz + 20.0 * n; break;                      // CSR SpMV: vals+cols, rowptr+x+y
+        case 0: *bytes = product(8); break;
         case 1: *bytes = 1290.0 * T + 632.0 * S; break;                     // element inputs + slot ids + 81/36 writes
         case 2: *bytes = 316.0 * T + 200.0 * S + 8.0 * n; break;            // element inputs + residual out
         case 3: *bytes = 8.0 * 81.0 * T + 8.0 * 36.0 * S + 12.0 * nnz; break;   // element blocks in, CSR values + map out
-        case 4: *bytes = 12.0 * nnz + 20.0 * n + 24.0 * n + 16.0 * n; break;    // SpMV + block-Jacobi apply
-        case 6: *bytes = 4.0 * (8.0 * nnz + 32.0 * n); break;   // ~4 level-0 matrix passes (coarse levels extra)
-        case 5: *bytes = 8.0 * nnz + 12.0 * n + 12.0 * n + 8.0 * n; break;   // FP32 SpMV + FP32 block apply
-        case 7: *bytes = 8.0 * nnz + 12.0 * n; break;                        // FP32 values + cols, x and y
+        case 4: *bytes = sweep(8); break;
+        case 5: *bytes = sweep(4); break;
+        case 6: *bytes = 4.0 * sweep(4); break;   // 4 level-0 matrix passes (coarse levels extra)
+        case 7: *bytes = product(4); break;
         case 8: *bytes = (double)(m->small_m32 > 0 ? m->small_m32 : m->gm_cycle_b32.m); break;   // iterations of the cycle (not bytes)
         case 9: *bytes = 4.0 * (double)m->p_rtot + 12.0 * m->p_nentries; break;   // FP32 inverse rows + residuals
     }
