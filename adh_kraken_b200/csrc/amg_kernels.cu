@@ -445,7 +445,10 @@ __global__ void __launch_bounds__(kAmgCoarsest, 1) k_coarsest_op(int n, const in
     if (mine) {
         const double x[3] = {x0, x1, x2};
 #pragma unroll
-        for (int v = 0; v < 3; v++) { op64[(size_t)(3 * i + v) * m + j] = x[v]; op32[(size_t)(3 * i + v) * m + j] = (float)x[v]; }
+        for (int v = 0; v < 3; v++) {
+            if (op64) op64[(size_t)(3 * i + v) * m + j] = x[v];
+            op32[(size_t)(3 * i + v) * m + j] = (float)x[v];
+        }
     }
 }
 
@@ -630,7 +633,7 @@ void patch_invert(const BlockCSR& A, const PatchDev& P, const double* vals, int 
 }
 
 // ---------------------------------------------------------------- host side
-void amg_setup(const BlockCSR& A, const AmgHost& H, const AssemblyMaps& maps, const double* vals, cudaStream_t st) {
+void amg_setup(const BlockCSR& A, const AmgHost& H, const AssemblyMaps& maps, const double* vals, bool fp32, cudaStream_t st) {
     k_amg_dinv0<<<nb(A.nnodes, 128), 128, 0, st>>>(A, vals, H.dinv0_64, H.patch.flag);
     for (int l = 1; l < H.nlev; l++) {
         const AmgLevel& C = H.lev[l];
@@ -647,7 +650,8 @@ void amg_setup(const BlockCSR& A, const AmgHost& H, const AssemblyMaps& maps, co
         k_cast32<<<1184, 256, 0, st>>>(9L * C.nb, C.val64, C.val32);
         k_cast32<<<1184, 256, 0, st>>>(9L * C.n, C.dinv64, C.dinv32);
     }
-    if (H.cl.ctas > 0) {   // (the FP64 form is read where the cluster starts at level 0, the FP32 form anywhere)
+    // FP64 cycles read the operator only where the cluster starts at level 0 (op64 is null elsewhere)
+    if (H.cl.ctas > 0 && (H.cl.lo == 0 || fp32)) {
         const AmgLevel& C = H.lev[H.nlev - 1];
         k_coarsest_op<<<3 * C.n, kAmgCoarsest, 0, st>>>(C.n, C.bptr, C.bcol, C.val64, C.dinv64, kAmgOmega, kAmgCoarseSweeps,
                                                         H.cl.op64, H.cl.op32);

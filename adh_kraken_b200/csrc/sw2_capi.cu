@@ -711,7 +711,8 @@ static int build_amg(sw2g_model* m);
 // preconditioner set-up on the scaled matrix (replaces prep_umfpack, bcgstab_solver.c:371)
 static int build_patches(sw2g_model* m, const double* vals);
 static void invalidate_graphs(sw2g_model* m);
-static int do_precond_setup(sw2g_model* m, const double* vals, int precond, int chunks = 0) {
+// fp32: the solve's cycles run in FP32
+static int do_precond_setup(sw2g_model* m, const double* vals, int precond, bool fp32, int chunks) {
     if (precond == SW2G_PC_AMG) {
         if (!m->amg_ready) TRY(build_amg(m));
         if (m->amg.patch.mode != chunks) {   // the placement is baked into the captured solver graphs
@@ -719,8 +720,9 @@ static int do_precond_setup(sw2g_model* m, const double* vals, int precond, int 
             m->amg.patch.mode = chunks;
         }
         {
-            ProfScope ps(m, 3, 1 + 4 * (m->amg.nlev - 1));
-            amg_setup(m->B, m->amg, m->A, vals, m->st);
+            const bool op = m->amg.cl.ctas > 0 && (m->amg.cl.lo == 0 || fp32);   // (as amg_setup)
+            ProfScope ps(m, 3, 2 + 4 * (m->amg.nlev - 1) + (op ? 1 : 0));
+            amg_setup(m->B, m->amg, m->A, vals, fp32, m->st);
             CKL();
         }
         return build_patches(m, vals);
@@ -867,8 +869,9 @@ static int build_amg(sw2g_model* m) {
     }
     if (A.lev[A.nlev - 1].n <= kAmgCoarsest) {   // the small levels in one cluster
         const size_t rows = 3 * (size_t)A.lev[A.nlev - 1].n;
-        TRY(dalloc(m, &A.cl.op64, rows * rows)); TRY(dalloc(m, &A.cl.op32, rows * rows));
         while (A.cl.lo < A.nlev - 1 && A.lev[A.cl.lo].n > kClusterNodes) A.cl.lo++;
+        if (A.cl.lo == 0) TRY(dalloc(m, &A.cl.op64, rows * rows));
+        TRY(dalloc(m, &A.cl.op32, rows * rows));
         A.cl.ctas = amg_cluster_ctas();
         std::vector<int> order = m->small_order;
         for (int l = 0; l < A.nlev - 1 && m->small.ctas > 0; l++) {
@@ -1586,7 +1589,7 @@ static int newton_device(sw2g_model* m, const sw2g_newton_opts& o_in, sw2g_newto
         TRY(do_jacobian(m, m->d_sol, m->d_sol_old, m->d_sol_older, m->d_wd, m->d_vals));
         CK(cudaMemsetAsync(m->d_dsol, 0, sizeof(double) * n, m->st));
         TRY(do_prepare(m, m->d_vals, m->d_res, m->d_dsol));
-        TRY(do_precond_setup(m, m->d_vals, o.precond, o.amg_chunks));
+        TRY(do_precond_setup(m, m->d_vals, o.precond, o.krylov_precision == 32, o.amg_chunks));
         int kit = 0, kst = 0, passes = 0;
         if (o.krylov_method == SW2G_KRYLOV_GMRES)
             TRY(solve_gmres(m, m->d_dsol, m->d_res, o, o.krylov_precision == 32, rmax, &kit, &passes, &kst));
@@ -1792,7 +1795,7 @@ extern "C" int sw2g_solve_linear_sys_bcgstab(sw2g_model* m, double* x, const dou
     CK(cudaMemcpyAsync(m->d_res, b, sizeof(double) * n, cudaMemcpyHostToDevice, m->st));
     CK(cudaMemcpyAsync(m->d_dsol, x, sizeof(double) * n, cudaMemcpyHostToDevice, m->st));
     CK(cudaMemcpyAsync(m->d_scale, scale_vect, sizeof(double) * n, cudaMemcpyHostToDevice, m->st));
-    TRY(do_precond_setup(m, m->d_vals, precond));
+    TRY(do_precond_setup(m, m->d_vals, precond, false, 0));
     int it = 0, status = 0;
     TRY(solve64(m, m->d_dsol, m->d_res, precond, max_it, tol, &it, &status));
     CK(cudaMemcpyAsync(x, m->d_dsol, sizeof(double) * n, cudaMemcpyDeviceToHost, m->st));
@@ -1955,7 +1958,7 @@ extern "C" int sw2g_time_kernel(sw2g_model* m, int which, int reps, double* avg_
     const double nnz = m->nnz, n = m->n, T = m->T, S = m->S;
     if (which >= 4) {   // the AMG sweeps
         if (!m->amg_ready) TRY(build_amg(m));
-        amg_setup(m->B, m->amg, m->A, m->d_vals, m->st);
+        amg_setup(m->B, m->amg, m->A, m->d_vals, true, m->st);
     }
     if (which == 5 || which == 6 || which == 7 || which == 9) {
         TRY(alloc_fp32(m));

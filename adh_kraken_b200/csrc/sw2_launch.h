@@ -169,7 +169,8 @@ constexpr int kClusterNodes = 2048;         // levels of at most this many nodes
 struct ClusterPlan {
     int ctas = 0;                           // CTAs of the cluster; 0: a kernel per pass and level
     int lo = 0;                             // first level in the cluster
-    double* op64 = nullptr; float* op32 = nullptr;   // [(3n)^2] the coarsest level's operator, written by amg_setup
+    // [(3n)^2] the coarsest level's operator, written by amg_setup; op64 only where lo is 0
+    double* op64 = nullptr; float* op32 = nullptr;
 };
 struct AmgHost {
     int nlev = 0;                       // levels including level 0
@@ -201,8 +202,8 @@ template <> struct AmgBuf<float> {
     static float* r(const AmgLevel& L) { return L.r32; }
 };
 int amg_cluster_ctas();                     // CTAs of the cluster on the current device, 0: not available
-// numeric set-up from the scaled level-0 matrix (FP64, plus FP32 copies); writes H.patch.flag
-void amg_setup(const BlockCSR& A, const AmgHost& H, const AssemblyMaps& maps, const double* vals, cudaStream_t st);
+// numeric set-up from the scaled level-0 matrix (FP64, plus FP32 copies; fp32: FP32 cycles follow); writes H.patch.flag
+void amg_setup(const BlockCSR& A, const AmgHost& H, const AssemblyMaps& maps, const double* vals, bool fp32, cudaStream_t st);
 // inverts the chunk blocks of the current patch build (nchunks from the host build)
 void patch_invert(const BlockCSR& A, const PatchDev& P, const double* vals, int nchunks, cudaStream_t st);
 // one level-0 smoothing sweep y = x + w Dinv (b - A x) (FP64; kernel timing)
