@@ -54,7 +54,9 @@ struct ProfRec { int cls; cudaEvent_t a, b; };
 // A GMRES cycle as captured graphs: segments of kGmSegment steps (the first with the cycle's start) and the end.  The
 // host looks at the stop flag between segments, so that a cycle that converges early does not replay the steps
 // left as empty launches: those were 400 of 600 steps of a 125k-triangle solve with GMRES(100), 1.3 us a launch, 10 of
-// 49 ms; a look costs ~15 us.  Cycles of up to kGmSegment + 7 steps stay whole.
+// 49 ms; a look costs ~15 us.  A step of the 2116-node basin with cycles of 26 / 30 / 32 / 40 steps takes 6.41 / 6.29 / 6.28 / 6.28 ms
+// in segments and 6.41 / 6.50 / 6.62 / 7.05 whole, so only cycles of one segment are; at 10,000 nodes the two are within 3 %
+// up to 32 steps, and at 63,000 within the runs' scatter.
 static const int kGmSegment = 25;
 struct CycleGraph {
     std::vector<cudaGraphExec_t> seg;
@@ -1199,7 +1201,7 @@ static int build_cycle(sw2g_model* m, CycleGraph* C, const PrecondOp<VT>& op, co
                        int mres) {
     if (C->m == mres && C->precond == op.kind) return SW2G_OK;
     C->clear();
-    const int n = m->n, seg = mres <= kGmSegment + 7 ? mres : kGmSegment;
+    const int n = m->n, seg = std::min(mres, kGmSegment);
     const size_t ld = gm_ld(n);
     for (int first = 0; first <= mres; first += seg) {   // the last round captures the end
         const bool end = first >= mres;
