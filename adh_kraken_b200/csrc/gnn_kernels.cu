@@ -589,9 +589,12 @@ static constexpr size_t fwd_smem(int in, int npt) { return sizeof(float) * ((siz
 static constexpr size_t bwd_smem(int in, int out, int npt) { return sizeof(float) * ((size_t)((out + 3) & ~3) * in + (size_t)16 * npt * (H + 4)); }
 static constexpr size_t narrow_smem(int in) { return sizeof(float) * ((size_t)in * NARROW + (size_t)NARROW_NODES * (in + 1)); }
 }
-// Tiles of 128 nodes from one per SM on; below that tiles of 16 nodes, which spread a small graph over more SMs
-// (1600 nodes, forward of all layers: 242 us with 64-node tiles, 47 us with 16).
-static bool wide_tiles(int n, int sms) { return (long)n >= 128L * sms; }
+// Tiles of 128 nodes, or of 16, which spread a small graph over more SMs, but read shared memory three times as often for a
+// multiply-add.  The line is where the two cross: one wide tile for two SMs where the products weigh (256 -> 64 forward, 16 and
+// 128 nodes: 26.8 and 28.8 us at 6000, 37.0 and 28.8 at 10,000, 56 and 29 at 18,900; with gradients 42 and 44, 58 and 52, 79 and 56),
+// one per SM in narrow layers (8 -> 64 forward: 6.3 and 9.3 us at 6000, 8.3 and 9.4 at 14,000, 10.3 and 9.4 at 18,900, 13.5 and
+// 10.4 at 30,000).
+static bool wide_tiles(int n, int in, int sms) { return (long)n >= (in > H ? 64L : 128L) * sms; }
 
 extern "C++" {
 template <int NPT>
@@ -618,7 +621,7 @@ int sw2n_dense_fwd(int n, int in, int out, const void* W_bf16, const float* b, c
     const int vec = (aligned16(X) ? VEC_X : 0) | (out % 4 == 0 && aligned16(Y) && aligned16(Z) && aligned16(R) ? VEC_OUT : 0) |
                     (in % 8 == 0 && aligned16(W) ? VEC_W : 0);
     const int sms = num_sms();
-    return wide_tiles(n, sms) ? run_dense_fwd<8>(n, in, out, W, b, X, R, act, Z, Y, vec, sms, st)
+    return wide_tiles(n, in, sms) ? run_dense_fwd<8>(n, in, out, W, b, X, R, act, Z, Y, vec, sms, st)
                               : run_dense_fwd<1>(n, in, out, W, b, X, R, act, Z, Y, vec, sms, st);
 }
 
@@ -642,7 +645,7 @@ int sw2n_dense_bwd(int n, int in, int out, const void* W_bf16, const float* X, c
     const __nv_bfloat16* W = (const __nv_bfloat16*)W_bf16;
     const int sms = num_sms(), vx = (aligned16(dX) ? VEC_OUT : 0) |
                                          (out % 4 == 0 && aligned16(dY) && aligned16(Z) && aligned16(dZ) ? VEC_IN : 0);
-    const bool ok = wide_tiles(n, sms) ? run_dense_bwd_x<8>(n, in, out, W, Z, dY, act, dZ, dX, vx, sms, st)
+    const bool ok = wide_tiles(n, in, sms) ? run_dense_bwd_x<8>(n, in, out, W, Z, dY, act, dZ, dX, vx, sms, st)
                                        : run_dense_bwd_x<1>(n, in, out, W, Z, dY, act, dZ, dX, vx, sms, st);
     if (!ok) return -2;
     const int nparts = nb(n, nodes_per_block);
