@@ -2027,8 +2027,8 @@ extern "C" int sw2g_time_kernel(sw2g_model* m, int which, int reps, double* avg_
 // variant keeps it in a file-scope device array of a fixed size instead, so a
 // call allocates nothing.  Every GPU that loads the library holds this array
 // (about 9.5 MB) until the process exits.
-constexpr int kNoAllocMaxElems = 1 << 17;   // triangles + boundary segments
-constexpr int kNoAllocMaxNodes = 1 << 17;
+constexpr int kNoAllocMaxElems = 1 << 17;   // triangles + boundary segments: the array's size
+constexpr int kNoAllocMaxNodes = 1 << 17;   // the call's stated limit; nothing here is sized by it
 constexpr int kNoAllocMaxDevices = 64;
 static __device__ __align__(256) double g_na_elem_resid[9 * (size_t)kNoAllocMaxElems];
 // the array's device address, looked up once per device (host code may not use the array's
@@ -2063,8 +2063,8 @@ extern "C" int sw2g_assemble_residual_noalloc(sw2g_model* m, const double* d_sol
                                               const double* d_sol_older, double* d_residual) {
     NEED(m && d_sol && d_sol_old && d_sol_older && d_residual, "sw2g_assemble_residual_noalloc: null argument");
     if (m->Etot > kNoAllocMaxElems || m->V > kNoAllocMaxNodes) {
-        g_err = "sw2g_assemble_residual_noalloc: the mesh has more than 131072 elements or nodes (the size of its "
-                "fixed work arrays); use sw2g_assemble_residual";
+        g_err = "sw2g_assemble_residual_noalloc: the mesh has more than 131072 elements (the size of its fixed work array) "
+                "or 131072 nodes; use sw2g_assemble_residual";
         return SW2G_ERR_ARG;
     }
     NoAllocScratch S{};

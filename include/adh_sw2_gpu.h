@@ -212,12 +212,13 @@ int sw2g_grid_mass(sw2g_model *m, const double *sol, double density, double dt, 
  * steps).  No counterpart in the reference.  The call allocates nothing: its work
  * array is a fixed-size device array inside the library (about 9.5 MB, held by every
  * GPU that loads it until the process exits), so the mesh may have at most 131072
- * elements (triangles + segments) and 131072 nodes; larger meshes get SW2G_ERR_ARG.
+ * elements (triangles + segments), and also at most 131072 nodes (a limit of the call, not
+ * of the array); larger meshes get SW2G_ERR_ARG.
  * d_sol, d_sol_old, d_sol_older [ndofs] and d_residual [ndofs] are device pointers on
  * the model's device; the step parameters come from sw2g_set_step.  The model's device
  * (the one current at sw2g_create) must be the current device when this is called
- * (SW2G_ERR_ARG otherwise).  The first call on a device looks the arrays' device
- * addresses up (once per device); make it before any stream capture.  Every call shares the arrays, so calls that overlap on the GPU
+ * (SW2G_ERR_ARG otherwise).  The first call on a device looks the array's device
+ * address up (once per device); make it before any stream capture.  Every call shares the array, so calls that overlap on the GPU
  * (other models, streams or host threads) race; the call returns after its kernels
  * have finished on the model's stream. */
 int sw2g_assemble_residual_noalloc(sw2g_model *m, const double *d_sol, const double *d_sol_old,
